@@ -71,6 +71,16 @@ template <class R> struct TablesView {
 
 template <class R> BTAM_HD R rmin(R a, R b) { return a < b ? a : b; }
 
+// a b + c in one rounding on the device: the expressions that several kernels
+// must agree on to the last bit leave no contraction to the compiler's choice.
+template <class R> BTAM_HD R mad(R a, R b, R c) {
+#if defined(__CUDA_ARCH__)
+  return fma(a, b, c);
+#else
+  return a * b + c;
+#endif
+}
+
 // Segment index m = min(int(x / dx), n - 1) (cubic-spline.cpp:89-90).  In
 // FP64 the index is the reference's: x times 1/dx truncates to the same
 // integer as the rounded quotient unless it lies within 1e-9 of a knot, and
@@ -94,7 +104,7 @@ template <class R> BTAM_HD int seg_index(R x, R dx, R inv_dx, int n) {
 template <class R>
 BTAM_HD void spline_vd(const SplineView<R> &s, R r, R &v, R &dv) {
   const int m = seg_index<R>(r, s.dx, s.inv_dx, s.n);
-  R p = rmin(r - (R)m * s.dx, s.dx);
+  R p = rmin(mad(-(R)m, s.dx, r), s.dx);
 #if defined(__CUDA_ARCH__)
   Coef4<R> k;
   if (sizeof(R) == 4) {
@@ -108,7 +118,7 @@ BTAM_HD void spline_vd(const SplineView<R> &s, R r, R &v, R &dv) {
 #else
   Coef4<R> k = s.c[m];
 #endif
-  v = k.a + (k.b + (k.c + k.d * p) * p) * p;
+  v = mad(mad(mad(k.d, p, k.c), p, k.b), p, k.a);
   dv = k.b + ((R)2 * k.c + (R)3 * k.d * p) * p;
 }
 
@@ -139,6 +149,10 @@ template <class R> struct RadialView {
   const R *pr;
   R dx, inv_dx;
   int n;
+  // the blocks again with the 32-byte pieces of the records placed for the
+  // kernels' gathers (uw_piece, pr_piece); device views only
+  const R *uwx = nullptr;
+  const R *prx = nullptr;
   // the uw block again, laid out as the shared-memory kernels stage it
   // (halves swapped where uw_swapped says), for one bulk copy; may be null
   const R *uws = nullptr;
@@ -162,13 +176,13 @@ BTAM_HD int rho_off(int pk, int c) { return (pk == 2 && c == 1) ? 8 : 4; }
 // p = min(s - m dx, dx).
 template <class R> BTAM_HD int seg_of(const RadialView<R> &T, R s, R &p) {
   const int m = seg_index<R>(s, T.dx, T.inv_dx, T.n);
-  p = rmin(s - (R)m * T.dx, T.dx);
+  p = rmin(mad(-(R)m, T.dx, s), T.dx);
   return m;
 }
 
 // Cubic a + (b + (c + d p) p) p and its derivative b + (2c + 3d p) p.
 template <class R> BTAM_HD R cub_v(const R *k, R p) {
-  return k[0] + (k[1] + (k[2] + k[3] * p) * p) * p;
+  return mad(mad(mad(k[3], p, k[2]), p, k[1]), p, k[0]);
 }
 template <class R> BTAM_HD void cub_vd(const R *k, R p, R &v, R &dv) {
   v = cub_v(k, p);
@@ -275,7 +289,7 @@ template <class R> struct V3 {
 };
 template <class R> BTAM_HD V3<R> mk3(R x, R y, R z) { return V3<R>{x, y, z}; }
 template <class R> BTAM_HD R dot3(const V3<R> &a, const V3<R> &b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z;
+  return mad(a.z, b.z, mad(a.y, b.y, a.x * b.x));
 }
 template <class R> BTAM_HD R comp(const V3<R> &a, int k) {
   return k == 0 ? a.x : (k == 1 ? a.y : a.z);
@@ -307,10 +321,10 @@ template <class R> struct Dual {
 
 template <class R, class S> BTAM_HD Dual<R> dual_of(const S *a, const S *l) {
   Dual<R> D;
-  S tr = l[0] + l[1] + l[2];
-  for (int k = 0; k < 3; ++k) D.a[k] = (R)(0.5 * a[k]);
-  for (int k = 0; k < 3; ++k) D.d[k] = (R)(0.5 * l[k] - tr / 6.0);
-  for (int k = 0; k < 3; ++k) D.o[k] = (R)(0.5 * l[3 + k]);
+  const S tr6 = (l[0] + l[1] + l[2]) / (S)6;
+  for (int k = 0; k < 3; ++k) D.a[k] = (R)((S)0.5 * a[k]);
+  for (int k = 0; k < 3; ++k) D.d[k] = (R)((S)0.5 * l[k] - tr6);
+  for (int k = 0; k < 3; ++k) D.o[k] = (R)((S)0.5 * l[3 + k]);
   return D;
 }
 
@@ -362,10 +376,83 @@ BTAM_HD void norm_inv(float s2, float &s, float &inv) {
   s = s2 * inv;
 }
 
-// The uw record of pair kind pk, segment m: a read-only global load, or a
+// Where a 32-byte piece of a record lies in uwx / prx.  A gather of random
+// records costs the L1 data pipe one cycle per piece that falls on the same
+// quarter of a 128-byte line; where every lane reads the same piece of its
+// record and records are 64 or 128 bytes, the plain layout puts all pieces on
+// two quarters or one (27 and 32 cycles a request measured, against 19 over all
+// four), so the pieces of a record are rotated with its index:
+//   64-byte records (FP64 uw, and pr of the same-species kinds; FP32 pr of
+//     Mg-H): pieces 0, 1 swapped on every other line;
+//   128-byte records (FP64 pr of Mg-H): piece c at (c + m) mod 4.
+// 32-byte records (FP32 uw) lie on all four quarters already.
+// Measured on 27,000 sites (3.6 M directed pairs), with the moment records
+// placed the same way (mom_at), plain against placed: FP64 pair rule 405 ->
+// 350 us, pass 1 545 -> 518, pass 2 591 -> 528; FP32C 151 -> 148, 211 -> 197,
+// 222 -> 210.
+BTAM_HD int rec64_piece(int r, int c) { return c ^ ((r >> 1) & 1); }
+BTAM_HD int rec128_piece(int m, int c) { return (c + m) & 3; }
+
+// The uw record of pair kind pk, segment m: read-only global loads, or a
 // shared load when the view's uw block is staged in shared memory.
-template <class R> BTAM_HD void ld_uw(const RadialView<R> &T, int pk, int m, R (&k)[8]) {
+BTAM_HD void ld_uw(const RadialView<float> &T, int pk, int m, float (&k)[8]) {
   ld8(uw_rec(T, pk, m), k);
+}
+BTAM_HD void ld_uw(const RadialView<double> &T, int pk, int m, double (&k)[8]) {
+#if defined(__CUDA_ARCH__)
+  const int r = T.n * pk + m;
+  const double *q = T.uwx + (size_t)kUWStride * r;
+  double u[4], w[4];
+  ld4(q + 4 * rec64_piece(r, 0), u);
+  ld4(q + 4 * rec64_piece(r, 1), w);
+  for (int c = 0; c < 4; ++c) {
+    k[c] = u[c];
+    k[4 + c] = w[c];
+  }
+#else
+  ld8(uw_rec(T, pk, m), k);
+#endif
+}
+// Cubics of phi (k[0..3]) and of the pr record's first rho (k[4..7]: the kind's
+// species, or Mg), and of H in a Mg-H record (h).
+BTAM_HD void ld_pr(const RadialView<float> &T, int pk, int m, float (&k)[8]) {
+#if defined(__CUDA_ARCH__)
+  // same-species kinds: 32-byte records; Mg-H: 64 bytes, pieces swapped
+  ld8(pk == 2 ? T.prx + (size_t)16 * T.n + 16 * (size_t)m + 8 * rec64_piece(m, 0)
+              : T.prx + (size_t)8 * (T.n * pk + m),
+      k);
+#else
+  ld8(pr_rec(T, pk, m), k);
+#endif
+}
+BTAM_HD void ld_pr(const RadialView<double> &T, int pk, int m, double (&k)[8]) {
+#if defined(__CUDA_ARCH__)
+  const int r = T.n * pk + m;
+  const double *q = T.prx + (pk == 2 ? (size_t)16 * (T.n + m) : (size_t)8 * r);
+  double a[4], b[4];
+  ld4(q + 4 * (pk == 2 ? rec128_piece(m, 0) : rec64_piece(r, 0)), a);
+  ld4(q + 4 * (pk == 2 ? rec128_piece(m, 1) : rec64_piece(r, 1)), b);
+  for (int c = 0; c < 4; ++c) {
+    k[c] = a[c];
+    k[4 + c] = b[c];
+  }
+#else
+  ld8(pr_rec(T, pk, m), k);
+#endif
+}
+BTAM_HD void ld_pr_h(const RadialView<float> &T, int m, float (&h)[4]) {
+#if defined(__CUDA_ARCH__)
+  ld4(T.prx + (size_t)16 * T.n + 16 * (size_t)m + 8 * rec64_piece(m, 1), h);
+#else
+  ld4(pr_rec(T, 2, m) + 8, h);
+#endif
+}
+BTAM_HD void ld_pr_h(const RadialView<double> &T, int m, double (&h)[4]) {
+#if defined(__CUDA_ARCH__)
+  ld4(T.prx + (size_t)16 * (T.n + m) + 4 * rec128_piece(m, 2), h);
+#else
+  ld4(pr_rec(T, 2, m) + 8, h);
+#endif
 }
 BTAM_HD void ld_uw(const RadialViewS<float> &T, int pk, int m, float (&k)[8]) {
   lds8(uw_rec<float>(T, pk, m), uw_swapped(T.n * pk + m), k);
@@ -400,9 +487,8 @@ BTAM_HD int geo_uw(Geo<R> &g, const V3<R> &r, const TV &T, int pk, R &p) {
 template <class R, bool D, bool WANT_I>
 BTAM_HD void pr_at(const RadialView<R> &T, int pk, int ci, int cj, int m, R p, R &ph, R &dph,
                    R &rj, R &drj, R &ri, R &dri) {
-  const R *base = pr_rec(T, pk, m);
   R k[8];
-  ld8(base, k);
+  ld_pr(T, pk, m, k);
   R r0 = (R)0, dr0 = (R)0, r1 = (R)0, dr1 = (R)0;
   if (D) {
     cub_vd(k, p, ph, dph);
@@ -414,7 +500,7 @@ BTAM_HD void pr_at(const RadialView<R> &T, int pk, int ci, int cj, int m, R p, R
   }
   if (pk == 2 && (cj == 1 || (WANT_I && ci == 1))) {
     R h[4];
-    ld4(base + 8, h);
+    ld_pr_h(T, m, h);
     if (D) cub_vd(h, p, r1, dr1);
     else r1 = cub_v(h, p);
   }
@@ -502,7 +588,7 @@ template <class R> BTAM_HD V3<R> dual_J(const Dual<R> &D, const Geo<R> &g) {
 // [u u' s + u^2 + 2/3 w w' s^3 + 4/3 w^2 s^2] r.
 template <class R> BTAM_HD R bff(const Geo<R> &g) {
   R s2 = g.s * g.s;
-  return (R)0.5 * g.u * g.u * s2 + g.w * g.w * s2 * s2 / (R)3;
+  return (R)0.5 * g.u * g.u * s2 + (R)(1.0 / 3.0) * g.w * g.w * s2 * s2;
 }
 template <class R> BTAM_HD R bff_grad_coef(const Geo<R> &g) {
   R s2 = g.s * g.s;
@@ -566,12 +652,20 @@ template <class R> BTAM_HD Dual<R> dual_from(const R (&h)[8], R o2) {
   D.o[0] = h[6]; D.o[1] = h[7]; D.o[2] = o2;
   return D;
 }
-template <class R, class S> BTAM_HD void store_dual(R *m, int k, const Dual<S> &D) {
-  R *h = m + 8 + 8 * k;
-  h[0] = (R)D.a[0]; h[1] = (R)D.a[1]; h[2] = (R)D.a[2];
-  h[3] = (R)D.d[0]; h[4] = (R)D.d[1]; h[5] = (R)D.d[2];
-  h[6] = (R)D.o[0]; h[7] = (R)D.o[1];
-  m[72 + k] = (R)D.o[2];
+// In the kernels' global arrays the 32-byte pieces of a site's record are
+// rotated with the site, for the reason given at rec64_piece: FP64 records are
+// five lines, so a piece would lie on the same quarter for every site; FP32
+// ones two and a half, so on two.  mom_x: a site's key; mom_at: where value c
+// of the record lies (key 0: the plain order, in shared and host memory).
+template <class R> BTAM_HD int mom_x(int site) { return sizeof(R) == 8 ? site & 3 : (site >> 1) & 1; }
+template <class R> BTAM_HD int mom_at(int c, int x) {
+  return sizeof(R) == 8 ? (((c >> 2) ^ x) << 2) | (c & 3) : (((c >> 3) ^ x) << 3) | (c & 7);
+}
+template <class R, class S> BTAM_HD void store_dual(R *m, int k, const Dual<S> &D, int x) {
+  const R h[8] = {(R)D.a[0], (R)D.a[1], (R)D.a[2], (R)D.d[0],
+                  (R)D.d[1], (R)D.d[2], (R)D.o[0], (R)D.o[1]};
+  for (int c = 0; c < 8; ++c) m[mom_at<R>(8 + 8 * k + c, x)] = h[c];
+  m[mom_at<R>(72 + k, x)] = (R)D.o[2];
 }
 
 // ---------------------------------------------------------------------------
@@ -846,16 +940,29 @@ template <class R> BTAM_HD R ld_ro(const R *p) {
 // are read once, with the record.
 template <class R, bool RO> struct MomRec {
   const R *m;
+  int x;  // key of the record's place (0: plain)
   R tail[8];
-  BTAM_HD explicit MomRec(const R *m_) : m(m_) {
-    if (RO) ld8(m + 72, tail);
-    else cp8(m + 72, tail);
+  BTAM_HD explicit MomRec(const R *m_, int x_ = 0) : m(m_), x(x_) { row(72, tail); }
+  BTAM_HD R scalar(int c) const {
+    return RO ? ld_ro(m + mom_at<R>(c, x)) : ld_plain(m + mom_at<R>(c, x));
   }
-  BTAM_HD R scalar(int c) const { return RO ? ld_ro(m + c) : ld_plain(m + c); }
+  // values [c, c + 8), c a multiple of 8
+  BTAM_HD void row(int c, R (&h)[8]) const {
+    if (!RO) cp8(m + c, h);
+    else if (sizeof(R) == 4) ld8(m + mom_at<R>(c, x), h);
+    else {
+      R lo[4], hi[4];
+      ld4(m + mom_at<R>(c, x), lo);
+      ld4(m + mom_at<R>(c + 4, x), hi);
+      for (int i = 0; i < 4; ++i) {
+        h[i] = lo[i];
+        h[4 + i] = hi[i];
+      }
+    }
+  }
   BTAM_HD Dual<R> dual(int k) const {
     R h[8];
-    if (RO) ld8(m + 8 + 8 * k, h);
-    else cp8(m + 8 + 8 * k, h);
+    row(8 + 8 * k, h);
     return dual_from(h, tail[k]);
   }
 };
@@ -1237,17 +1344,17 @@ constexpr double kUma = 103.4993333E-6;     // eV A^-2 ps^2 per amu
 // G0, 1: H, 2 + d: G(d)) and returns B(G(d), G(d)) for the G(d) duals;
 // site_scalars takes bgd = sum_d B(G(d), G(d)) (summed in d order) and does
 // the rest.
-template <class M> BTAM_HD double site_dual(const SiteSums &S, int k, M *mom) {
+template <class M> BTAM_HD double site_dual(const SiteSums &S, int k, M *mom, int x = 0) {
   const double *a = k == 0 ? S.g0a : (k == 1 ? S.ha : S.gda[k - 2]);
   const double *l = k == 0 ? S.g0l : (k == 1 ? S.hl : S.gdl[k - 2]);
-  if (mom) store_dual(mom, k, dual_of<double, double>(a, l));
+  if (mom) store_dual(mom, k, dual_of<double, double>(a, l), x);
   return k >= 2 ? bself(a, l) : 0.0;
 }
 
 template <class M>
 BTAM_HD void site_scalars(const SiteSums &S, double bgd, const SplineView<double> &emb,
                           double xi, int code, double beta, double gamma, double sigma,
-                          double mass, SiteResult &res, M *mom) {
+                          double mass, SiteResult &res, M *mom, int x = 0) {
   const double rho = kW6 * S.rho;
   double F, dF;
   spline_vd(emb, rho, F, dF);
@@ -1269,10 +1376,10 @@ BTAM_HD void site_scalars(const SiteSums &S, double bgd, const SplineView<double
   double gx = (code == 1) ? gamma * (xi > 0.9999 ? 0.9999 : xi) : 0.0;
   res.S0 = -logZ + beta * (1.0 / (2.0 * beta) + V0) - gx;
   if (mom) {
-    mom[0] = (M)(xi * dF);
-    mom[1] = (M)((code == 1 ? xi : 1.0) * dF);
-    mom[2] = (M)beta;
-    for (int c = 3; c < 8; ++c) mom[c] = (M)0;
+    mom[mom_at<M>(0, x)] = (M)(xi * dF);
+    mom[mom_at<M>(1, x)] = (M)((code == 1 ? xi : 1.0) * dF);
+    mom[mom_at<M>(2, x)] = (M)beta;
+    for (int c = 3; c < 8; ++c) mom[mom_at<M>(c, x)] = (M)0;
   }
 }
 

@@ -570,14 +570,14 @@ pass1_kernel(const EvalArgs<R> a) {
   // epilogue: lanes 0..7 of the group form the record's eight duals, lane 0
   // the rest
   double b = 0.0;
-  if (act && sl < 8) b = site_dual(ss[warp * SPW + half], sl, mom);
+  if (act && sl < 8) b = site_dual(ss[warp * SPW + half], sl, mom, mom_x<R>(i));
   double bgd = 0.0;
 #pragma unroll
   for (int d = 0; d < 6; ++d) bgd += __shfl_sync(0xffffffffu, b, gbase + 2 + d);
   if (act && sl == 0) {
     SiteResult res;
     site_scalars(ss[warp * SPW + half], bgd, a.emb[ci], xi, ci, xbi.y, a.gamma[i], qi.w,
-                 a.mass[ci], res, mom);
+                 a.mass[ci], res, mom, mom_x<R>(i));
     a.rho[i] = res.rho;
     a.V0[i] = res.V0;
     a.S0[i] = res.S0;
@@ -613,7 +613,7 @@ pass2_kernel(const EvalArgs<R> a) {
     continue;
   }
   const R *mu_g = a.mom + (size_t)u * kMomStride;
-  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[c];
+  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[mom_at<R>(c, mom_x<R>(u))];
   __syncwarp();
   const MomRec<R, false> mu(mu_s[warp]);
   const double4 qu = a.pos[u];
@@ -626,7 +626,7 @@ pass2_kernel(const EvalArgs<R> a) {
     if (xbj.x < kMinOcc) continue;
     const int o = a.owner[j];
     const double4 qj = a.pos[j];
-    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride);
+    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride, mom_x<R>(o));
     Pass2Out<R> out;
     out.gq[0] = out.gq[1] = out.gq[2] = out.gs = out.gx = (R)0;
     pass2_pair<R>(a.T, pair_vec<R>(qu, qj), (R)qu.w, (R)qj.w, (R)xu, (R)xbj.x, cu,
@@ -677,7 +677,7 @@ mf_stress_kernel(const EvalArgs<R> a, double *W0) {
     continue;
   }
   const R *mu_g = a.mom + (size_t)u * kMomStride;
-  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[c];
+  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[mom_at<R>(c, mom_x<R>(u))];
   __syncwarp();
   const MomRec<R, false> mu(mu_s[warp]);
   const double4 qu = a.pos[u];
@@ -689,7 +689,7 @@ mf_stress_kernel(const EvalArgs<R> a, double *W0) {
     if (xbj.x < kMinOcc) continue;
     const int o = a.owner[j];
     const double4 qj = a.pos[j];
-    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride);
+    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride, mom_x<R>(o));
     Pass2Out<R> out;
     out.gq[0] = out.gq[1] = out.gq[2] = out.gs = out.gx = (R)0;
     const V3<R> r0 = pair_vec<R>(qu, qj);
@@ -739,7 +739,7 @@ mf_pair_terms_kernel(const EvalArgs<R> a, double *self, double *slot) {
     continue;
   }
   const R *mu_g = a.mom + (size_t)u * kMomStride;
-  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[c];
+  for (int c = lane; c < kMomStride; c += 32) mu_s[warp][c] = mu_g[mom_at<R>(c, mom_x<R>(u))];
   __syncwarp();
   const MomRec<R, false> mu(mu_s[warp]);
   const double4 qu = a.pos[u];
@@ -753,7 +753,7 @@ mf_pair_terms_kernel(const EvalArgs<R> a, double *self, double *slot) {
     if (!(xbj.x < kMinOcc)) {
       const int o = a.owner[j];
       const double4 qj = a.pos[j];
-      const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride);
+      const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride, mom_x<R>(o));
       Pass2Parts<R> P;
       pass2_pair_parts<R>(a.T, pair_vec<R>(qu, qj), (R)qu.w, (R)qj.w, (R)xu, (R)xbj.x, cu,
                           a.code[j], mu.scalar(0), mj.scalar(0), mj.scalar(1), mu, mj, P);
@@ -805,8 +805,8 @@ __device__ __forceinline__ void pass2u_one(const EvalArgs<R> &a, const TV &T, in
   if (su.active && sj.active) {
     const int o = sj.owner;
     const double bu = su.beta, bj = sj.beta;
-    const MomRec<R, true> mu(a.mom + (size_t)u * kMomStride);
-    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride);
+    const MomRec<R, true> mu(a.mom + (size_t)u * kMomStride, mom_x<R>(u));
+    const MomRec<R, true> mj(a.mom + (size_t)o * kMomStride, mom_x<R>(o));
     Pass2Out<R> ou, oj;
     ou.gq[0] = ou.gq[1] = ou.gq[2] = ou.gs = ou.gx = (R)0;
     oj.gq[0] = oj.gq[1] = oj.gq[2] = oj.gs = oj.gx = (R)0;
@@ -999,8 +999,8 @@ __global__ void rho_nmf_kernel(int n, const double4 *pos, const double2 *xb, con
       double xj = xb[j].x;
       if (xj < kMinOcc) continue;
       double4 qj = pos[j];
-      double dx = qi.x - qj.x, dy = qi.y - qj.y, dz = qi.z - qj.z;
-      double r = sqrt(dx * dx + dy * dy + dz * dz);
+      const V3<double> d = pair_vec<double>(qi, qj);
+      double r = sqrt(dot3(d, d));
       acc += xj * spline_v(code[j] == 0 ? rmg : rh, r);
     }
   }

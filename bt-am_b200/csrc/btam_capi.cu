@@ -487,6 +487,23 @@ int btam_tables_load(const char *dir, btam_tables **out) {
     btam_tables_destroy(t);
     return cuda_status(e);
   }
+  const std::vector<double> x64 =
+      place_radial(r64, uw64, pr64, rn, rec64_piece, rec128_piece);
+  const std::vector<float> x32 = place_radial(r32, uw32, pr32, rn, rec64_piece, rec128_piece);
+  e = cudaMalloc(&t->radx64, x64.size() * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&t->radx32, x32.size() * sizeof(float));
+  if (e == cudaSuccess)
+    e = cudaMemcpy(t->radx64, x64.data(), x64.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(t->radx32, x32.data(), x32.size() * sizeof(float), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    btam_tables_destroy(t);
+    return cuda_status(e);
+  }
+  t->r64.uwx = t->radx64 + uw64[0];
+  t->r64.prx = t->radx64 + pr64[0];
+  t->r32.uwx = t->radx32 + uw32[0];
+  t->r32.prx = t->radx32 + pr32[0];
   t->r64.uw = t->rad64 + uw64[0];
   t->r64.pr = t->rad64 + pr64[0];
   t->r32.uw = t->rad32 + uw32[0];
@@ -545,6 +562,8 @@ void btam_tables_destroy(btam_tables *t) {
   if (t->d32) cudaFree(t->d32);
   if (t->rad64) cudaFree(t->rad64);
   if (t->rad32) cudaFree(t->rad32);
+  if (t->radx64) cudaFree(t->radx64);
+  if (t->radx32) cudaFree(t->radx32);
   if (t->uws32) cudaFree(t->uws32);
   if (t->uws64) cudaFree(t->uws64);
   delete t;

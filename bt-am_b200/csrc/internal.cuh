@@ -26,8 +26,8 @@ struct btam_tables {
   TablesView<double> v64;
   TablesView<float> v32;
   // the radial tables as the kernels' per-segment records
-  double *rad64 = nullptr;
-  float *rad32 = nullptr;
+  double *rad64 = nullptr, *radx64 = nullptr;  // plain; pieces placed for gathers
+  float *rad32 = nullptr, *radx32 = nullptr;
   float *uws32 = nullptr;  // the FP32 uw block in its shared-memory layout
   double *uws64 = nullptr;  // the FP64 uw block in its shared-memory layout
   RadialView<double> r64;

@@ -115,4 +115,32 @@ bool pack_radial(const HostTables &T, std::vector<R> &buf, size_t off_uw[3], siz
   return true;
 }
 
+// The packed records with their 32-byte pieces at the places of rec64_piece
+// and rec128_piece: n segments, E values per piece (4 doubles or 8 floats).
+// piece64(r, c), piece128(m, c): the place of piece c of a record.
+template <class R, class P64, class P128>
+std::vector<R> place_radial(const std::vector<R> &src, const size_t off_uw[3],
+                            const size_t off_pr[3], int n, P64 piece64, P128 piece128) {
+  std::vector<R> out = src;
+  const size_t E = 32 / sizeof(R);
+  auto move = [&](size_t at, int from, int to) {
+    for (size_t e = 0; e < E; ++e) out[at + E * to + e] = src[at + E * from + e];
+  };
+  for (int m = 0; m < n; ++m) {
+    for (int c = 0; c < 2; ++c) {
+      if (sizeof(R) == 8)
+        for (int pk = 0; pk < 3; ++pk) {
+          const int r = n * pk + m;
+          move(off_uw[0] + 8 * (size_t)r, c, piece64(r, c));
+          if (pk < 2) move(off_pr[0] + 8 * (size_t)r, c, piece64(r, c));
+        }
+      else
+        move(off_pr[2] + 16 * (size_t)m, c, piece64(m, c));
+    }
+    if (sizeof(R) == 8)
+      for (int c = 0; c < 4; ++c) move(off_pr[2] + 16 * (size_t)m, c, piece128(m, c));
+  }
+  return out;
+}
+
 }  // namespace btam
