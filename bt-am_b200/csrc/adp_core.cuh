@@ -602,7 +602,7 @@ template <class R> BTAM_HD Dual<R> dual_feat(const Geo<R> &g, R X) {
   R hu = (R)0.5 * X * g.u, hw = (R)0.5 * X * g.w;
   R s2 = g.s * g.s;
   D.a[0] = hu * g.r.x; D.a[1] = hu * g.r.y; D.a[2] = hu * g.r.z;
-  R t = X * g.w * s2 / (R)6;
+  R t = (R)(1.0 / 6.0) * X * g.w * s2;
   D.d[0] = hw * g.r.x * g.r.x - t;
   D.d[1] = hw * g.r.y * g.r.y - t;
   D.d[2] = hw * g.r.z * g.r.z - t;
@@ -680,7 +680,7 @@ template <class R> BTAM_HD R bpair_r(const Feat<R> &x, const Feat<R> &y) {
   R lm = x.l[0] * y.l[0] + x.l[1] * y.l[1] + x.l[2] * y.l[2] +
          (R)2 * (x.l[3] * y.l[3] + x.l[4] * y.l[4] + x.l[5] * y.l[5]);
   R t1 = x.l[0] + x.l[1] + x.l[2], t2 = y.l[0] + y.l[1] + y.l[2];
-  return (R)0.5 * ab + (R)0.5 * lm - t1 * t2 / (R)6;
+  return (R)0.5 * ab + (R)0.5 * lm - (R)(1.0 / 6.0) * t1 * t2;
 }
 
 // The 12-point pair rule of an owned pair (u, j), once for both passes and

@@ -107,6 +107,35 @@ constexpr int kPass2Variants = 6;  // shapes (4,-), (4,3), (4,4), (4,5), (8,2), 
 constexpr int kPass2UVariants = 7;
 constexpr int kPersistent = 8;
 constexpr int kUndirected = 16;
+// Neither pinned nor tuned yet: the library picks (default_variants).
+constexpr int kAutoVariant = -1;
+// Launch variants of a system or batch of n real sites that has none: the
+// undirected kernels (their pair buffer permitting), which look each pair's
+// pair rule up once and take pass 2 from one evaluation per pair.  Directed
+// (0, 0) against undirected, both passes, FP64: 99 -> 68 us at 350 sites, 310
+// -> 155 at 2,916, 1345 -> 585 at 10,920, 7600 -> 2900 at 95,331; FP32C: 62 ->
+// 56, 165 -> 86, 622 -> 254, 3317 -> 1167.
+// Shapes: a warp per site while the sites leave warps idle (pass 1 at 350 and
+// 605 sites 26 and 27 us against 37 and 40 for half a warp, at 2,916 sites 75
+// against 56); the persistent grid once it has several trips (95,331 sites:
+// 1075 against 1098 us).
+inline void default_variants(bool fp64, int n, int *v1, int *v2) {
+  if (n < 1500) {
+    *v1 = kUndirected;
+    *v2 = kUndirected | (fp64 ? 0 : 6);
+  } else if (fp64) {
+    *v1 = kUndirected | 5 | (n < 20000 ? 0 : kPersistent);
+    *v2 = kUndirected | 6 | kPersistent;
+  } else {
+    *v1 = kUndirected | (n < 6000 ? 5 : (2 | kPersistent));
+    *v2 = kUndirected | 6 | kPersistent;
+  }
+}
+// Whether a pair buffer of `need` bytes may be taken without being asked for:
+// up to 256 MB or what the library pool holds unused, else at most a quarter
+// of the device memory that is free; and not while the stream is being
+// captured (an allocation would belong to the graph).
+bool may_take(size_t need, cudaStream_t st);
 inline bool valid_variants(int v1, int v2) {
   if (v1 < 0 || v2 < 0 || (v1 & ~(2 * kUndirected - 1)) != 0 ||
       (v2 & ~(2 * kUndirected - 1)) != 0)

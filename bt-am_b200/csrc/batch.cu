@@ -137,9 +137,9 @@ struct btam_batch {
   double *mom64 = nullptr;
   float *mom32 = nullptr;
   int *err = nullptr;
-  // launch variants per arithmetic form (0 FP64, 1 FP32C); persistent grids
-  // unless btam_batch_autotune finds a full grid faster
-  int variant1[2] = {kPersistent, kPersistent}, variant2[2] = {kPersistent, kPersistent};
+  // launch variants per arithmetic form (0 FP64, 1 FP32C), as
+  // btam_batch_autotune or btam_batch_set_variants left them
+  int variant1[2] = {kAutoVariant, kAutoVariant}, variant2[2] = {kAutoVariant, kAutoVariant};
   // instantiated graph per form and the variants it was captured with
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   int exec_v1[2] = {-1, -1}, exec_v2[2] = {-1, -1};
@@ -205,6 +205,23 @@ int batch_pbuf(btam_batch *b, size_t elem) {
   BTAM_TRY(dalloc(b->pbuf, b->st, need));
   b->pbuf_bytes = need;
   return BTAM_OK;
+}
+
+// The launch variants of the batch's next evaluation in form f: the pinned or
+// tuned ones, else default_variants if their pair buffer is there or may be
+// taken, else the directed kernels on persistent grids.
+void batch_pick_variants(btam_batch *b, int f, int *v1, int *v2) {
+  *v1 = b->variant1[f];
+  *v2 = b->variant2[f];
+  if (*v1 != kAutoVariant) return;
+  *v1 = *v2 = kPersistent;
+  if (take_pbuf(b->pbuf, b->pbuf_bytes, b->pbuf_elem,
+                pbuf_values(b->n_pairs > 0 ? b->n_pairs : 1, b->n_own),
+                f == 0 ? sizeof(double) : sizeof(float), b->st)) {
+    default_variants(f == 0, b->n_real, v1, v2);
+    *v1 |= kPersistent;
+    *v2 |= kPersistent;
+  }
 }
 
 int batch_read_err(btam_batch *b) {
@@ -382,10 +399,11 @@ int batch_build(btam_batch *b) {
 }
 
 // Enqueues one evaluation of every system: pass 1, pass 2, per-system totals.
-template <class R> cudaError_t enqueue_eval(btam_batch *b, int form, R *mom, const RadialView<R> &T) {
+template <class R>
+cudaError_t enqueue_eval(btam_batch *b, int v1, int v2, R *mom, const RadialView<R> &T) {
   EvalArgs<R> a = batch_args<R>(b, mom, T);
-  cudaError_t e = launch_pass1(a, b->st, b->variant1[form], b->variant2[form]);
-  if (e == cudaSuccess) e = launch_pass2(a, b->st, b->variant2[form]);
+  cudaError_t e = launch_pass1(a, b->st, v1, v2);
+  if (e == cudaSuccess) e = launch_pass2(a, b->st, v2);
   if (e == cudaSuccess)
     e = launch_seg_totals(b->n_sys, b->seg, b->V0, b->S0, b->Rq, b->Rs, b->Rx, b->totals,
                           b->totals + 4 * (size_t)b->n_sys, b->st);
@@ -403,8 +421,9 @@ int ensure_moments(btam_batch *b, int precision) {
 // when the launch variants changed since the last capture).
 int ensure_graph(btam_batch *b, int precision) {
   const int f = precision == BTAM_FP64 ? 0 : 1;
-  if (b->exec[f] && b->exec_v1[f] == b->variant1[f] && b->exec_v2[f] == b->variant2[f] &&
-      b->exec_pbuf[f] == b->pbuf)
+  int v1, v2;
+  batch_pick_variants(b, f, &v1, &v2);
+  if (b->exec[f] && b->exec_v1[f] == v1 && b->exec_v2[f] == v2 && b->exec_pbuf[f] == b->pbuf)
     return BTAM_OK;
   if (b->exec[f]) {
     cudaGraphExecDestroy(b->exec[f]);
@@ -412,8 +431,8 @@ int ensure_graph(btam_batch *b, int precision) {
   }
   cudaGraph_t g = nullptr;
   BTAM_TRY(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeRelaxed));
-  cudaError_t e = f == 0 ? enqueue_eval<double>(b, 0, b->mom64, b->T->r64)
-                         : enqueue_eval<float>(b, 1, b->mom32, b->T->r32);
+  cudaError_t e = f == 0 ? enqueue_eval<double>(b, v1, v2, b->mom64, b->T->r64)
+                         : enqueue_eval<float>(b, v1, v2, b->mom32, b->T->r32);
   cudaError_t e2 = cudaStreamEndCapture(b->st, &g);
   if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[f], g, 0);
@@ -422,8 +441,8 @@ int ensure_graph(btam_batch *b, int precision) {
     b->exec[f] = nullptr;
     return cuda_status(e);
   }
-  b->exec_v1[f] = b->variant1[f];
-  b->exec_v2[f] = b->variant2[f];
+  b->exec_v1[f] = v1;
+  b->exec_v2[f] = v2;
   b->exec_pbuf[f] = b->pbuf;
   return BTAM_OK;
 }
@@ -557,8 +576,11 @@ int batch_round(btam_batch *b, const BatchXfer &t, const cudaEvent_t *ready, int
   int st = ensure_moments(b, precision);
   if (st != BTAM_OK) return st;
   b->masked = true;
-  const cudaError_t ev = precision == BTAM_FP64 ? enqueue_eval<double>(b, 0, b->mom64, b->T->r64)
-                                                : enqueue_eval<float>(b, 1, b->mom32, b->T->r32);
+  int v1, v2;
+  batch_pick_variants(b, precision == BTAM_FP64 ? 0 : 1, &v1, &v2);
+  const cudaError_t ev = precision == BTAM_FP64
+                             ? enqueue_eval<double>(b, v1, v2, b->mom64, b->T->r64)
+                             : enqueue_eval<float>(b, v1, v2, b->mom32, b->T->r32);
   b->masked = false;
   BTAM_TRY(ev);
   batch_scatter_kernel<<<grid, 256, 0, b->st>>>(t, b->rho, b->V0, b->S0, b->Rq, b->Rs, b->Rx,

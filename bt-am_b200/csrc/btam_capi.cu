@@ -300,9 +300,24 @@ int ensure_pbuf(btam_system *s, size_t elem) {
       pbuf_values(s->n_pairs > 0 ? s->n_pairs : 1, s->n_own) * elem;
   s->pbuf_elem = elem;
   if (need <= s->pbuf_bytes) return BTAM_OK;
+  s->pbuf_bytes = 0;
   BTAM_TRY(dalloc(s->pbuf, s->st, need));
   s->pbuf_bytes = need;
   return BTAM_OK;
+}
+
+// The launch variants of the system's next evaluation in form f (0 FP64, 1
+// FP32C): the pinned or tuned ones, else default_variants if their pair
+// buffer is there or may be taken, else the directed kernels, which need none.
+void pick_variants(btam_system *s, int f, int *v1, int *v2) {
+  *v1 = s->variant1[f];
+  *v2 = s->variant2[f];
+  if (*v1 != kAutoVariant) return;
+  *v1 = *v2 = 0;
+  const size_t elem = f == 0 ? sizeof(double) : sizeof(float);
+  if (take_pbuf(s->pbuf, s->pbuf_bytes, s->pbuf_elem,
+                pbuf_values(s->n_pairs > 0 ? s->n_pairs : 1, s->n_own), elem, s->st))
+    default_variants(f == 0, s->n_real, v1, v2);
 }
 
 // the pipelined state evaluations' buffers, events and copy streams
@@ -323,20 +338,22 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
   if (precision != BTAM_FP64 && precision != BTAM_FP32C) return BTAM_ERR_ARG;
   if (s->batcher) return batcher_eval(s, precision);  // a served job: one shared launch
   const size_t nm = (size_t)s->n_real * kMomStride;
+  int v1, v2;
+  pick_variants(s, precision == BTAM_FP64 ? 0 : 1, &v1, &v2);
   if (precision == BTAM_FP64) {
     if (!s->mom64) BTAM_TRY(dalloc(s->mom64, s->st, nm));
     EvalArgs<double> a = eval_args<double>(s, s->mom64, s->T->r64);
     a.x_only = x_only;
     a.recs_ready = x_only && recs_ready;
-    BTAM_TRY(launch_pass1(a, s->st, s->variant1[0], s->variant2[0]));
-    BTAM_TRY(launch_pass2(a, s->st, s->variant2[0]));
+    BTAM_TRY(launch_pass1(a, s->st, v1, v2));
+    BTAM_TRY(launch_pass2(a, s->st, v2));
   } else {
     if (!s->mom32) BTAM_TRY(dalloc(s->mom32, s->st, nm));
     EvalArgs<float> a = eval_args<float>(s, s->mom32, s->T->r32);
     a.x_only = x_only;
     a.recs_ready = x_only && recs_ready;
-    BTAM_TRY(launch_pass1(a, s->st, s->variant1[1], s->variant2[1]));
-    BTAM_TRY(launch_pass2(a, s->st, s->variant2[1]));
+    BTAM_TRY(launch_pass1(a, s->st, v1, v2));
+    BTAM_TRY(launch_pass2(a, s->st, v2));
   }
   BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->totals + 4,
                           s->st));
@@ -368,6 +385,29 @@ cudaMemPool_t device_pool() {
     pools[dev] = p;
   }
   return pools[dev];
+}
+
+bool may_take(size_t need, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaMemPool_t pool = device_pool();
+  unsigned long long used = 0, held = 0;
+  size_t spare = 0;
+  if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess)
+    spare = held > used ? (size_t)(held - used) : 0;
+  // the query of the free memory takes 0.3 to 18 ms: not for what the pool
+  // holds unused, nor for a small buffer
+  if (need <= spare || need <= ((size_t)256 << 20)) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return need <= (free_b + spare) / 4;
 }
 
 const TablesView<double> &tables_view64(const btam_tables *t) { return t->v64; }
@@ -800,7 +840,13 @@ int btam_neighbors_build(btam_system *s, int all_sites) {
   BTAM_TRY(launch_pair_links(n, s->offs, s->idx, s->owner, s->rev, s->slot_own, s->cnt,
                              s->own_off, s->own_p, s->own_u, s->own_cap, &s->n_own, s->scratch,
                              s->st));
-  if (s->pbuf_elem > 0) {  // a rebuilt list may be longer than the slot buffer
+  // a rebuilt list may be longer than the pair buffer: pinned undirected
+  // variants need it, the defaults take it again at the next evaluation
+  bool pinned = false;
+  for (int f = 0; f < 2; ++f)
+    pinned = pinned || (s->variant1[f] != kAutoVariant &&
+                        ((s->variant1[f] | s->variant2[f]) & kUndirected) != 0);
+  if (pinned && s->pbuf_elem > 0) {
     int st2 = ensure_pbuf(s, s->pbuf_elem);
     if (st2 != BTAM_OK) return st2;
   }
@@ -907,7 +953,10 @@ int btam_mf_eval_async(btam_system *s, int precision) {
 }
 
 int btam_mf_eval_x(btam_system *s, int precision) {
-  return enqueue_eval(s, precision, true, false);
+  // the occupancy gradients alone for variants that were asked for; a system
+  // left to the defaults gets the full evaluation
+  const bool pinned = s && s->variant1[precision == BTAM_FP64 ? 0 : 1] != kAutoVariant;
+  return enqueue_eval(s, precision, pinned, false);
 }
 
 }  // extern "C"
@@ -1229,20 +1278,22 @@ int btam_mf_eval_profile(btam_system *s, int precision, double ms[5]) {
   cudaEvent_t ev[6];
   for (auto &e : ev) BTAM_TRY(cudaEventCreate(&e));
   const size_t nm = (size_t)s->n_real * kMomStride;
-  cudaError_t e = cudaEventRecord(ev[0], s->st);
   const int f = precision == BTAM_FP64 ? 0 : 1;
+  int v1, v2;
+  pick_variants(s, f, &v1, &v2);
+  cudaError_t e = cudaEventRecord(ev[0], s->st);
   if (precision == BTAM_FP64) {
     if (!s->mom64 && e == cudaSuccess) e = dalloc(s->mom64, s->st, nm);
     EvalArgs<double> a = eval_args<double>(s, s->mom64, s->T->r64);
-    if (e == cudaSuccess) e = launch_pass1(a, s->st, s->variant1[f], s->variant2[f], ev[1]);
+    if (e == cudaSuccess) e = launch_pass1(a, s->st, v1, v2, ev[1]);
     if (e == cudaSuccess) e = cudaEventRecord(ev[2], s->st);
-    if (e == cudaSuccess) e = launch_pass2(a, s->st, s->variant2[f], ev[3]);
+    if (e == cudaSuccess) e = launch_pass2(a, s->st, v2, ev[3]);
   } else {
     if (!s->mom32 && e == cudaSuccess) e = dalloc(s->mom32, s->st, nm);
     EvalArgs<float> a = eval_args<float>(s, s->mom32, s->T->r32);
-    if (e == cudaSuccess) e = launch_pass1(a, s->st, s->variant1[f], s->variant2[f], ev[1]);
+    if (e == cudaSuccess) e = launch_pass1(a, s->st, v1, v2, ev[1]);
     if (e == cudaSuccess) e = cudaEventRecord(ev[2], s->st);
-    if (e == cudaSuccess) e = launch_pass2(a, s->st, s->variant2[f], ev[3]);
+    if (e == cudaSuccess) e = launch_pass2(a, s->st, v2, ev[3]);
   }
   if (e == cudaSuccess) e = cudaEventRecord(ev[4], s->st);
   if (e == cudaSuccess)

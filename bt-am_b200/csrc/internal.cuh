@@ -72,9 +72,9 @@ struct btam_system {
   float *mom32 = nullptr;
   int *err = nullptr;
   DeviceScratch scratch;
-  // kernel block shapes per arithmetic form (index 0 FP64, 1 FP32C), chosen
-  // by btam_autotune
-  int variant1[2] = {0, 0}, variant2[2] = {0, 0};
+  // kernel launch variants per arithmetic form (index 0 FP64, 1 FP32C), as
+  // btam_autotune or btam_set_variants left them
+  int variant1[2] = {kAutoVariant, kAutoVariant}, variant2[2] = {kAutoVariant, kAutoVariant};
   int cnt_cap = 0;
   // diffusive graph and master-equation state
   bool dmd_ready = false;
@@ -222,6 +222,28 @@ template <class T> inline cudaError_t dalloc(T *&p, cudaStream_t st, size_t coun
 template <class T> inline void dfree(T *&p, cudaStream_t st) {
   if (p) cudaFreeAsync(p, st);
   p = nullptr;
+}
+
+// Pair buffer for the default variants: `values` values of at least `elem`
+// bytes, if they are there or may be taken (may_take).  The buffer that is
+// there stays when they are not.
+inline bool take_pbuf(char *&pbuf, size_t &bytes, size_t &held_elem, size_t values, size_t elem,
+                      cudaStream_t st) {
+  if (elem < held_elem) elem = held_elem;
+  const size_t need = values * elem;
+  if (need > bytes) {
+    char *p = nullptr;
+    if (!may_take(need, st)) return false;
+    if (dalloc(p, st, need) != cudaSuccess) {
+      cudaGetLastError();  // nothing is left to report: other kernels run
+      return false;
+    }
+    dfree(pbuf, st);
+    pbuf = p;
+    bytes = need;
+  }
+  held_elem = elem;
+  return true;
 }
 
 // Synchronous copies ordered on a stream (the memory may come from the

@@ -314,6 +314,9 @@ void run_job(btam_server *srv, Job *job) {
   } else if (st == BTAM_OK && !sp.plain) {
     st = btam_set_variants(s, BTAM_FP32C, kServeVariant1[1], kServeVariant2[1]);
     if (st == BTAM_OK) st = btam_set_variants(s, BTAM_FP64, kServeVariant1[0], kServeVariant2[0]);
+  } else if (st == BTAM_OK) {  // the plain two-pass pair
+    st = btam_set_variants(s, BTAM_FP32C, 0, 0);
+    if (st == BTAM_OK) st = btam_set_variants(s, BTAM_FP64, 0, 0);
   }
   if (st == BTAM_OK) {
     r.t_start = since(srv->t0);

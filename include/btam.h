@@ -248,8 +248,8 @@ int btam_mf_eval_async(btam_system *s, int precision);
  * (MgHx-mf-V-bulk.cpp:2102-2325) assembled as in btam_mf_eval.  These are
  * the master equation's chemical potentials; btam_dmd_step takes them this
  * way and keeps the pair rule's position-only sums between its steps.  The
- * directed kernel variants and a served job's evaluations compute the full
- * residuals instead. */
+ * directed kernel variants, a system whose variants are neither tuned nor
+ * pinned and a served job's evaluations compute the full residuals instead. */
 int btam_mf_eval_x(btam_system *s, int precision);
 int btam_results_copy(btam_system *s, double *rho, double *V0, double *S0,
                       double *Rq, double *Rs, double *Rx, double *totals);
@@ -262,7 +262,11 @@ int btam_system_sync(btam_system *s);
  * (shape index, plus 8 for the persistent grid).  A given variant is bitwise
  * reproducible; the grid (full or persistent) never changes a bit, while
  * two block shapes are separate compilations and may round differently in
- * the last bits (within the stated tolerance of the form). */
+ * the last bits (within the stated tolerance of the form).  A system (or
+ * batch) that is neither tuned nor pinned takes undirected shapes by its
+ * size, or the directed kernels (0, 0) where their pair buffer would be more
+ * than 256 MB and more than a quarter of the free device memory, cannot be
+ * had, or would have to be allocated inside a stream capture. */
 int btam_autotune(btam_system *s, int precision, int *pass1_variant, int *pass2_variant);
 /* Pins the launch variants of `precision` (as reported by btam_autotune),
  * for runs that must reproduce one another bit for bit. */
