@@ -331,8 +331,11 @@ void release_state_slots(btam_system *s);
 // the pair-rule kernel's four pass-1 sums are still those of the current
 // positions and widths (an earlier x_only evaluation in the same run of
 // master-equation steps made them), so pass 1 skips that kernel.  A served
-// job's evaluation goes to the server's batcher in full.
-static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_ready) {
+// job's evaluation goes to the server's batcher in full.  totals: also the
+// system's totals (the solvers form their own sums and complete the totals
+// once, at the end).
+static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_ready,
+                        bool totals = true) {
   if (!s) return BTAM_ERR_ARG;
   if (!s->built) return BTAM_ERR_NOT_BUILT;
   if (precision != BTAM_FP64 && precision != BTAM_FP32C) return BTAM_ERR_ARG;
@@ -355,8 +358,9 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
     BTAM_TRY(launch_pass1(a, s->st, v1, v2));
     BTAM_TRY(launch_pass2(a, s->st, v2));
   }
-  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->totals + 4,
-                          s->st));
+  if (totals)
+    BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals,
+                           s->totals + 4, s->st));
   return BTAM_OK;
 }
 
@@ -1490,22 +1494,66 @@ namespace {
 
 // Evaluation followed by the relaxation view of it: z, g, F and |R|^2.
 struct RelaxVecs {
-  double *z, *g, *p, *z0, *g0, *work, *tmp, *fterm, *rterm, *ones, *scal, *rho, *alpha;
-  double *S[16], *Y[16];
+  double *z, *g, *p, *z0, *g0;
+  double *part;     // partial sums of relax_gather
+  unsigned *count;  // its block count (0 between calls)
+  double *out;      // lbfgs_step's four, then relax_gather's three
+  double *tmp;      // 8 scratch scalars
+  double *rho;      // 16
   RelaxBounds bd;
 };
+constexpr int kRelaxSmall = 64;  // doubles: out, tmp, rho, count and what follows
 
-int relax_eval(btam_system *s, int prec, RelaxVecs &v, double &f, double &r2) {
-  int st = btam_mf_eval_async(s, prec);
+// Lays the small arrays out behind the vectors, at b (3 n + kRelaxSmall
+// doubles), and clears the count.
+cudaError_t relax_small(btam_system *s, RelaxVecs &v, double *b) {
+  v.part = b;
+  v.out = b + 3 * (size_t)s->n_real;
+  v.tmp = v.out + 8;
+  v.rho = v.tmp + 8;
+  v.count = reinterpret_cast<unsigned *>(v.rho + 16);
+  return cudaMemsetAsync(v.count, 0, sizeof(double), s->st);
+}
+
+RelaxImages relax_images(const btam_system *s) {
+  RelaxImages im;
+  im.n = s->n_ghost;
+  im.owner = s->owner;
+  im.image = s->image;
+  im.box = s->box;
+  return im;
+}
+
+// The state to z0 + alpha p, alpha = scale times *alpha_dev (if given).
+cudaError_t relax_move(btam_system *s, const RelaxVecs &v, const double *z0, const double *p,
+                       double scale, const double *alpha_dev = nullptr) {
+  return relax_apply(s->n_real, s->xb, z0, p, scale, alpha_dev, v.bd, s->pos, relax_images(s),
+                     s->st);
+}
+
+// Evaluation of the state and the relaxation's view of it (z, g), with one
+// wait for its scalars: F, |R|^2 and the error bits, and (step) lbfgs_step's.
+int relax_eval(btam_system *s, int prec, RelaxVecs &v, double &f, double &r2,
+               double *step = nullptr) {
+  int st = enqueue_eval(s, prec, false, false, false);
   if (st != BTAM_OK) return st;
-  BTAM_TRY(relax_gather(s->n_real, s->pos, s->xb, s->V0, s->Rq, s->Rs, v.bd, v.z, v.g, v.fterm,
-                        v.rterm, v.scal, v.scal + 1, v.ones, s->st));
-  double h[2];
-  BTAM_TRY(cudaMemcpyAsync(h, v.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  st = read_err(s);
-  f = h[0];
-  r2 = h[1];
-  return st;
+  BTAM_TRY(relax_gather(s->n_real, s->pos, s->xb, s->V0, s->Rq, s->Rs, v.bd, v.z, v.g, v.part,
+                        v.count, s->err, v.out + 4, s->st));
+  double h[7];
+  BTAM_TRY(copy_sync(h, v.out, sizeof(h), cudaMemcpyDeviceToHost, s->st));
+  if (step)
+    for (int c = 0; c < 4; ++c) step[c] = h[c];
+  f = h[4];
+  r2 = h[5];
+  return status_from_bits((int)h[6]);
+}
+
+// The totals of the last evaluation (a served one brought its own).
+int relax_totals(btam_system *s) {
+  if (s->batcher) return BTAM_OK;
+  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->totals + 4,
+                         s->st));
+  return BTAM_OK;
 }
 
 double dev_dot(btam_system *s, RelaxVecs &v, int n, const double *a, const double *b) {
@@ -1514,11 +1562,6 @@ double dev_dot(btam_system *s, RelaxVecs &v, int n, const double *a, const doubl
   cudaMemcpyAsync(&h, v.tmp + 7, sizeof(double), cudaMemcpyDeviceToHost, s->st);
   cudaStreamSynchronize(s->st);
   return h;
-}
-
-__global__ void fill_kernel(int n, double v, double *a) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = v;
 }
 
 // g / beta per site: the N-GMRES residual in energy units
@@ -1570,9 +1613,9 @@ int relax_ngmres(btam_system *s, double tol, int max_iter, int m, const double *
                x_min = bounds ? bounds[2] : 0.01;
   if (!(sig_lo > 0.0 && sig_hi > sig_lo && x_min >= 0.0)) return BTAM_ERR_ARG;
   const int n = s->n_real, n4 = 4 * n;
-  // X F XM FM XA FA D, Xd[m] Fd[m] (n4 each), fterm rterm ones (n), scalars
+  // X F XM FM XA FA D, Xd[m] Fd[m] (n4 each), the small arrays, 40 dot products
   double *buf = nullptr;
-  BTAM_TRY(dalloc(buf, s->st, (size_t)(7 + 2 * m) * n4 + 3 * (size_t)n + 64));
+  BTAM_TRY(dalloc(buf, s->st, (size_t)(7 + 2 * m) * n4 + 3 * (size_t)n + kRelaxSmall + 40));
   double *X = buf, *F = buf + n4, *XM = buf + 2 * (size_t)n4, *FM = buf + 3 * (size_t)n4,
          *XA = buf + 4 * (size_t)n4, *FA = buf + 5 * (size_t)n4, *D = buf + 6 * (size_t)n4;
   std::vector<double *> Xd(m), Fd(m);
@@ -1581,26 +1624,15 @@ int relax_ngmres(btam_system *s, double tol, int max_iter, int m, const double *
     Fd[k] = buf + (size_t)(7 + m + k) * n4;
   }
   RelaxVecs v;
-  v.fterm = buf + (size_t)(7 + 2 * m) * n4;
-  v.rterm = v.fterm + n;
-  v.ones = v.rterm + n;
-  v.scal = v.ones + n;
-  v.tmp = v.scal + 2;  // 8 scratch scalars
-  double *dots = v.tmp + 8;  // up to 40 dot products
+  int st = cuda_status(relax_small(s, v, buf + (size_t)(7 + 2 * m) * n4));
+  double *dots = v.out + kRelaxSmall;
   v.bd.ls_lo = std::log(sig_lo);
   v.bd.ls_hi = std::log(sig_hi);
   v.bd.x_min = x_min;
-  fill_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(n, 1.0, v.ones);
-  int st = cuda_status(cudaGetLastError());
   if (st == BTAM_OK) st = cuda_status(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
   // state at z (with the bounds), then its evaluation into (Z, G)
   auto eval_at = [&](const double *z, double *Z, double *G, double &r2) -> int {
-    if (z) {
-      BTAM_TRY(relax_apply(n, s->xb, z, z, 0.0, v.bd, s->pos, s->st));
-      if (s->n_ghost > 0)
-        BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
-                                      s->box, s->st));
-    }
+    if (z) BTAM_TRY(relax_move(s, v, z, z, 0.0));
     v.z = Z;
     v.g = G;
     double f = 0.0;
@@ -1746,11 +1778,9 @@ int relax_ngmres(btam_system *s, double tol, int max_iter, int m, const double *
   if (st == BTAM_OK) {
     v.z = XM;
     v.g = FM;
-    st = cuda_status(relax_apply(n, s->xb, X, X, 0.0, v.bd, s->pos, s->st));
-    if (st == BTAM_OK && s->n_ghost > 0)
-      st = cuda_status(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner,
-                                            s->image, s->box, s->st));
+    st = cuda_status(relax_move(s, v, X, X, 0.0));
     if (st == BTAM_OK) st = relax_eval(s, BTAM_FP64, v, ff, r2f);
+    if (st == BTAM_OK) st = relax_totals(s);
   }
   dfree(buf, s->st);
   if (info) {
@@ -1784,8 +1814,9 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
                x_min = bounds ? bounds[2] : 0.01;
   if (!(sig_lo > 0.0 && sig_hi > sig_lo && x_min >= 0.0)) return BTAM_ERR_ARG;
   const int n = s->n_real, n4 = 4 * n;
-  // layout: z g p z0 g0 work (n4 each), S[m] Y[m] (n4 each), fterm rterm ones (n), small
-  const size_t need = (size_t)(6 + 2 * m) * n4 + 3 * (size_t)n + 64;
+  // layout: z g p z0 g0 and a spare (n4 each), S[m] Y[m] (n4 each), the small
+  // arrays; with m = 1 the size of btam_relax_newton's, which shares the block
+  const size_t need = (size_t)(6 + 2 * m) * n4 + 3 * (size_t)n + kRelaxSmall;
   if (!s->rv || s->relax_m < m) {
     BTAM_TRY(dalloc(s->rv, s->st, need));
     s->relax_m = m;
@@ -1793,24 +1824,20 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
   RelaxVecs v;
   double *b = s->rv;
   v.z = b; v.g = b + n4; v.p = b + 2 * n4; v.z0 = b + 3 * n4; v.g0 = b + 4 * n4;
-  v.work = b + 5 * n4;
-  for (int k = 0; k < m; ++k) {
-    v.S[k] = b + (size_t)(6 + k) * n4;
-    v.Y[k] = b + (size_t)(6 + m + k) * n4;
-  }
-  v.fterm = b + (size_t)(6 + 2 * m) * n4;
-  v.rterm = v.fterm + n;
-  v.ones = v.rterm + n;
-  v.scal = v.ones + n;
-  v.tmp = v.scal + 2;       // 8 scratch scalars
-  v.rho = v.tmp + 8;        // m
-  v.alpha = v.rho + 16;     // m
+  BTAM_TRY(relax_small(s, v, b + (size_t)(6 + 2 * m) * n4));
   v.bd.ls_lo = std::log(sig_lo);
   v.bd.ls_hi = std::log(sig_hi);
   v.bd.x_min = x_min;
-  fill_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(n, 1.0, v.ones);
-  BTAM_TRY(cudaGetLastError());
   BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
+  LbfgsStep step;
+  step.n4 = n4;
+  step.z = v.z; step.g = v.g; step.z0 = v.z0; step.g0 = v.g0;
+  step.S = b + (size_t)6 * n4;
+  step.Y = b + (size_t)(6 + m) * n4;
+  step.rho = v.rho;
+  step.xb = s->xb;
+  step.p = v.p;
+  step.out = v.out;
 
   int prec = (mode == 0) ? BTAM_FP64 : BTAM_FP32C;
   const double switch_tol = 1e-5;  // FP32C noise floor is ~1e-6
@@ -1818,47 +1845,39 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
   int evals = 0, it = 0, st;
   if ((st = relax_eval(s, prec, v, f, r2)) != BTAM_OK) return st;
   ++evals;
-  std::vector<int> order;
-  std::vector<double> rho_h(16, 0.0);
+  std::vector<int> order;  // history slots, newest last
+  int new_slot = -1;       // where the last step's pair goes
   bool stalled = false;
   for (; it < max_iter; ++it) {
     if (mode == 1 && prec == BTAM_FP32C && std::sqrt(r2) < switch_tol) {
       prec = BTAM_FP64;
       order.clear();
+      new_slot = -1;
       if ((st = relax_eval(s, prec, v, f, r2)) != BTAM_OK) return st;
       ++evals;
     }
     if (std::sqrt(r2) <= tol) break;
-    BTAM_TRY(lbfgs_direction(n4, v.g, v.S, v.Y, v.rho, order.data(), (int)order.size(), v.p,
-                             v.work, v.alpha, v.tmp, s->st));
-    double gp = dev_dot(s, v, n4, v.g, v.p);
-    if (!(gp < 0.0)) {  // not a descent direction: restart from steepest descent
-      order.clear();
-      BTAM_TRY(lbfgs_direction(n4, v.g, v.S, v.Y, v.rho, nullptr, 0, v.p, v.work, v.alpha, v.tmp,
-                               s->st));
-      gp = dev_dot(s, v, n4, v.g, v.p);
-    }
-    // first step of a history: move no q (A) or log sigma by more than 0.05;
-    // this step also seeds the curvature scale of the history
-    double alpha = 1.0;
-    if (order.empty()) {
-      absmax_kernel<<<1, 256, 0, s->st>>>(n4, s->xb, v.p, v.tmp + 6);
-      double pmax = 0.0;
-      BTAM_TRY(cudaMemcpyAsync(&pmax, v.tmp + 6, sizeof(double), cudaMemcpyDeviceToHost, s->st));
-      BTAM_TRY(cudaStreamSynchronize(s->st));
-      if (pmax > 0.05) alpha = 0.05 / pmax;
-    }
-    BTAM_TRY(cudaMemcpyAsync(v.z0, v.z, n4 * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
-    BTAM_TRY(cudaMemcpyAsync(v.g0, v.g, n4 * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
+    // the direction, its slope and the first trial's step length stay on the
+    // device; the host reads them with the first trial's evaluation
+    step.m_used = (int)order.size();
+    for (int t = 0; t < step.m_used; ++t) step.order[t] = order[t];
+    step.new_slot = new_slot;
+    BTAM_TRY(lbfgs_step(step, s->st));
     const double f0 = f, r20 = r2;
+    double gp = 0.0, alpha = 0.0, scale = 1.0;
     bool ok = false;
     for (int ls = 0; ls < 30; ++ls) {
-      BTAM_TRY(relax_apply(n, s->xb, v.z0, v.p, alpha, v.bd, s->pos, s->st));
-      if (s->n_ghost > 0)
-        BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
-                                      s->box, s->st));
-      if ((st = relax_eval(s, prec, v, f, r2)) != BTAM_OK) return st;
+      BTAM_TRY(relax_move(s, v, v.z0, v.p, scale, v.out + 1));
+      double h[4];
+      if ((st = relax_eval(s, prec, v, f, r2, h)) != BTAM_OK) return st;
       ++evals;
+      if (ls == 0) {
+        gp = h[0];
+        alpha = h[1];
+        if (new_slot >= 0 && h[3] > 1e-300) order.push_back(new_slot);
+        new_slot = -1;
+        if (h[2] != 0.0) order.clear();
+      }
       // Armijo decrease of F; once F's changes are below its rounding (about
       // 1e-7 relative in the FP32C form, 1e-13 in FP64), a step that lowers
       // the residual is accepted instead
@@ -1868,12 +1887,10 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
         break;
       }
       alpha *= 0.5;
+      scale *= 0.5;
     }
     if (!ok) {  // no decrease resolvable at this precision: restore and stop
-      BTAM_TRY(relax_apply(n, s->xb, v.z0, v.p, 0.0, v.bd, s->pos, s->st));
-      if (s->n_ghost > 0)
-        BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
-                                      s->box, s->st));
+      BTAM_TRY(relax_move(s, v, v.z0, v.p, 0.0));
       if (mode == 1 && prec == BTAM_FP32C) prec = BTAM_FP64;  // finish in FP64
       if ((st = relax_eval(s, prec, v, f, r2)) != BTAM_OK) return st;
       ++evals;
@@ -1882,22 +1899,11 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
         continue;
       }
       stalled = true;
-      (void)r20;
       break;
     }
-    // history pair (newest last, oldest dropped)
-    int slot = (int)order.size() < m ? (int)order.size() : order.front();
+    // slot of the step's pair (oldest dropped); the next direction makes it
+    new_slot = (int)order.size() < m ? (int)order.size() : order.front();
     if ((int)order.size() == m) order.erase(order.begin());
-    BTAM_TRY(lbfgs_push(n4, v.z, v.z0, v.g, v.g0, v.S[slot], v.Y[slot], v.tmp, s->st));
-    double sy = 0.0;
-    BTAM_TRY(cudaMemcpyAsync(&sy, v.tmp, sizeof(double), cudaMemcpyDeviceToHost, s->st));
-    BTAM_TRY(cudaStreamSynchronize(s->st));
-    if (sy > 1e-300) {
-      rho_h[slot] = 1.0 / sy;
-      BTAM_TRY(cudaMemcpyAsync(v.rho + slot, &rho_h[slot], sizeof(double), cudaMemcpyHostToDevice,
-                               s->st));
-      order.push_back(slot);
-    }
   }
   if (info) {
     info[0] = std::sqrt(r2);
@@ -1906,6 +1912,7 @@ int btam_relax(btam_system *s, int mode, double tol, int max_iter, int m, const 
     info[3] = f;
     info[4] = (std::sqrt(r2) <= tol) ? 1.0 : (stalled ? -1.0 : 0.0);
   }
+  if ((st = relax_totals(s)) != BTAM_OK) return st;
   BTAM_TRY(cudaStreamSynchronize(s->st));
   return BTAM_OK;
 }
@@ -1918,9 +1925,9 @@ int btam_relax_newton(btam_system *s, double tol, int max_newton, int max_cg,
                x_min = bounds ? bounds[2] : 0.01;
   if (!(sig_lo > 0.0 && sig_hi > sig_lo && x_min >= 0.0)) return BTAM_ERR_ARG;
   const int n = s->n_real, n4 = 4 * n;
-  // layout: z g p z0 g0 r d hd (n4 each), fterm rterm ones (n), small; the
-  // block of btam_relax with m = 1 has exactly this size
-  const size_t need = (size_t)8 * n4 + 3 * (size_t)n + 64;
+  // layout: z g p z0 g0 r d hd (n4 each), the small arrays; the block of
+  // btam_relax with m = 1 has exactly this size
+  const size_t need = (size_t)8 * n4 + 3 * (size_t)n + kRelaxSmall;
   if (!s->rv) {
     BTAM_TRY(dalloc(s->rv, s->st, need));
     s->relax_m = 1;
@@ -1929,24 +1936,13 @@ int btam_relax_newton(btam_system *s, double tol, int max_newton, int max_cg,
   double *b = s->rv;
   v.z = b; v.g = b + n4; v.p = b + 2 * n4; v.z0 = b + 3 * n4; v.g0 = b + 4 * n4;
   double *r = b + 5 * n4, *d = b + 6 * n4, *hd = b + 7 * n4;
-  v.work = nullptr;
-  v.fterm = b + (size_t)8 * n4;
-  v.rterm = v.fterm + n;
-  v.ones = v.rterm + n;
-  v.scal = v.ones + n;
-  v.tmp = v.scal + 2;
+  BTAM_TRY(relax_small(s, v, b + (size_t)8 * n4));
   v.bd.ls_lo = std::log(sig_lo);
   v.bd.ls_hi = std::log(sig_hi);
   v.bd.x_min = x_min;
-  fill_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(n, 1.0, v.ones);
-  BTAM_TRY(cudaGetLastError());
   BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
   auto move = [&](const double *z0, const double *p, double alpha) -> int {
-    BTAM_TRY(relax_apply(n, s->xb, z0, p, alpha, v.bd, s->pos, s->st));
-    if (s->n_ghost > 0)
-      BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
-                                    s->box, s->st));
-    return BTAM_OK;
+    return cuda_status(relax_move(s, v, z0, p, alpha));
   };
   double f, r2;
   int evals = 0, it = 0, cg_total = 0, st;
@@ -2046,6 +2042,7 @@ int btam_relax_newton(btam_system *s, double tol, int max_newton, int max_cg,
     info[4] = (std::sqrt(r2) <= tol) ? 1.0 : (stalled ? -1.0 : 0.0);
     info[5] = cg_total;
   }
+  if ((st = relax_totals(s)) != BTAM_OK) return st;
   BTAM_TRY(cudaStreamSynchronize(s->st));
   return BTAM_OK;
 }

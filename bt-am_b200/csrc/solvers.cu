@@ -14,32 +14,235 @@
 // Armijo line search; the vectors stay on the device, the host only reads
 // two scalars per line-search trial.  Converged when
 // sqrt(sum |R_q|^2 + R_sigma^2) <= tol.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <vector>
 
 #include "solvers.cuh"
+#include "topo_kernels.cuh"
 
 namespace btam {
 
 namespace {
 
-constexpr int kRB = 1024;  // threads of the single-block reductions
+constexpr int kRB = 1024;  // threads of the reduction blocks
 
-// Deterministic single-block reduction of sum a[i] * b[i] (fixed strides,
-// fixed tree).
+// Sum (or maximum) over the block of each thread's v, in every thread: fixed
+// shuffle trees, sh holds one value per warp.
+template <bool MAX> __device__ __forceinline__ double block_reduce(double v, double *sh) {
+  auto op = [](double a, double b) { return MAX ? fmax(a, b) : a + b; };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) sh[warp] = v;
+  __syncthreads();
+  v = sh[lane];  // kRB / 32 = 32 warps
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();  // sh is written again by the next reduction
+  return v;
+}
+
+// A cluster's reductions: every block leaves its value in every block's
+// shared memory and combines them in rank order.  Two sets of slots in turn,
+// so that one cluster barrier per reduction suffices: a slot is written again
+// two reductions later, past a barrier that every reader has reached.
+struct ClusterReduce {
+  static constexpr int kMax = 8;
+  double (*slots)[kMax];  // [2][kMax], shared
+  double *sh;             // 32, shared
+  int rank, size, turn = 0;
+  // every block runs before its slots are written, none leaves before that
+  __device__ __forceinline__ void begin() const {
+    if (size > 1) cooperative_groups::this_cluster().sync();
+  }
+  __device__ __forceinline__ void end() const { begin(); }
+  template <bool MAX> __device__ __forceinline__ double reduce(double v) {
+    v = block_reduce<MAX>(v, sh);
+    if (size == 1) return v;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    double *own = slots[turn];
+    if ((int)threadIdx.x < size) cl.map_shared_rank(own, threadIdx.x)[rank] = v;
+    cl.sync();
+    double r = own[0];
+    for (int k = 1; k < size; ++k) r = MAX ? fmax(r, own[k]) : r + own[k];
+    turn ^= 1;
+    return r;
+  }
+  __device__ __forceinline__ double sum(double v) { return reduce<false>(v); }
+  __device__ __forceinline__ double max(double v) { return reduce<true>(v); }
+};
+
+// Blocks of a cluster for vectors of n values: one block holds up to four
+// values a thread without the cluster's barriers; above that eight SMs read
+// the vectors (one block streams about 0.1 TB/s: a dot product of 108,000
+// values takes 13.5 us in one block).
+inline int cluster_of(int n) { return n <= 4 * kRB ? 1 : ClusterReduce::kMax; }
+
+template <class... KA, class... A>
+cudaError_t launch_cluster(void (*k)(KA...), int size, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(kRB);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, KA(args)...);
+}
+
+// Sum a[i] * b[i] over one cluster (fixed strides, fixed tree).
 __global__ void __launch_bounds__(kRB) dot_kernel(int n, const double *a, const double *b,
                                                   double *out) {
-  __shared__ double sh[kRB];
+  __shared__ double sh[32], slots[2][ClusterReduce::kMax];
+  const int size = gridDim.x, rank = blockIdx.x;
+  ClusterReduce R{slots, sh, rank, size};
+  R.begin();
   double v = 0.0;
-  for (int i = threadIdx.x; i < n; i += kRB) v += a[i] * b[i];
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = kRB / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
+  for (int i = rank * kRB + threadIdx.x; i < n; i += size * kRB) v += a[i] * b[i];
+  v = R.sum(v);
+  if (rank == 0 && threadIdx.x == 0) *out = v;
+  R.end();
+}
+
+// One L-BFGS direction (LbfgsStep): the newest pair from the last step, the
+// two-loop recursion, and what the line search needs of p, in one launch of
+// one cluster.  It replaces 7 launches per pair of the history and 6 more; each
+// was a few microseconds of latency with one reduction in it.  What bounds it
+// is the latency of its 2 m + 4 reductions, about a microsecond each over the
+// cluster.  Relaxation calls with this, the images moved with their owners and
+// the host reading once per trial, before and after: 15 iterations of 605
+// sites 5.36 -> 2.33 ms, 10 of 27,000 sites 23.4 -> 20.4 ms.
+__global__ void __launch_bounds__(kRB) lbfgs_step_kernel(const LbfgsStep a) {
+  __shared__ double sh[32], slots[2][ClusterReduce::kMax];
+  const int size = gridDim.x, rank = blockIdx.x, n4 = a.n4;
+  const int i0 = rank * kRB + threadIdx.x, step = size * kRB;
+  ClusterReduce R{slots, sh, rank, size};
+  R.begin();
+  auto S = [&](int k) { return a.S + (size_t)k * n4; };
+  auto Y = [&](int k) { return a.Y + (size_t)k * n4; };
+  // the pair of the last step; kept if its curvature is positive
+  int used = a.m_used;
+  int order[LbfgsStep::kMax + 1];
+  for (int t = 0; t < used; ++t) order[t] = a.order[t];
+  double sy = 0.0, yy = 0.0;
+  bool fresh = false;  // sy and yy are those of the newest pair in use
+  double rho_new = 0.0;
+  if (a.new_slot >= 0) {
+    double *s = S(a.new_slot), *y = Y(a.new_slot);
+    double v = 0.0, w = 0.0;
+    for (int i = i0; i < n4; i += step) {
+      const double ds = a.z[i] - a.z0[i], dy = a.g[i] - a.g0[i];
+      s[i] = ds;
+      y[i] = dy;
+      v += dy * ds;
+      w += dy * dy;
+    }
+    sy = R.sum(v);
+    yy = R.sum(w);
+    if (sy > 1e-300) {
+      rho_new = 1.0 / sy;
+      order[used++] = a.new_slot;
+      fresh = true;
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+      if (fresh) a.rho[a.new_slot] = rho_new;
+      a.out[3] = sy;
+    }
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  auto rho_of = [&](int k) { return fresh && k == a.new_slot ? rho_new : a.rho[k]; };
+  double *q = a.p;  // the recursion runs in p's buffer, each thread on its own values
+  double alpha[LbfgsStep::kMax + 1];
+  {
+    double v = 0.0;  // s . q of the newest pair
+    const double *s = used > 0 ? S(order[used - 1]) : nullptr;
+    for (int i = i0; i < n4; i += step) {
+      const double gi = a.g[i];
+      q[i] = gi;
+      if (s) v += s[i] * gi;
+    }
+    for (int t = used - 1; t >= 0; --t) {
+      const int k = order[t];
+      const double al = rho_of(k) * R.sum(v);
+      alpha[t] = al;
+      const double *y = Y(k), *sn = t > 0 ? S(order[t - 1]) : nullptr;
+      v = 0.0;
+      for (int i = i0; i < n4; i += step) {
+        const double qi = q[i] + -1.0 * al * y[i];
+        q[i] = qi;
+        if (sn) v += sn[i] * qi;
+      }
+    }
+  }
+  if (used > 0) {
+    const int k = order[used - 1];
+    if (!fresh) {  // H0 = (s.y)/(y.y) I of an older pair
+      double v = 0.0, w = 0.0;
+      const double *s = S(k), *y = Y(k);
+      for (int i = i0; i < n4; i += step) {
+        v += s[i] * y[i];
+        w += y[i] * y[i];
+      }
+      sy = R.sum(v);
+      yy = R.sum(w);
+    }
+    const double h0 = yy > 0.0 ? sy * (1.0 / yy) : 1.0;
+    double v = 0.0;  // y . q of the oldest pair
+    const double *y = Y(order[0]);
+    for (int i = i0; i < n4; i += step) {
+      const double qi = q[i] * h0;
+      q[i] = qi;
+      v += y[i] * qi;
+    }
+    for (int t = 0; t < used; ++t) {
+      const int j = order[t];
+      const double c = __dsub_rn(alpha[t], __dmul_rn(rho_of(j), R.sum(v)));
+      const double *s = S(j), *yn = t + 1 < used ? Y(order[t + 1]) : nullptr;
+      v = 0.0;
+      for (int i = i0; i < n4; i += step) {
+        const double qi = q[i] + 1.0 * c * s[i];
+        q[i] = qi;
+        if (yn) v += yn[i] * qi;
+      }
+    }
+  }
+  // p = -q, g.p, the largest move in unscaled units; the step's start
+  double gp = 0.0, mx = 0.0;
+  for (int i = i0; i < n4; i += step) {
+    const double pi = -q[i], gi = a.g[i];
+    q[i] = pi;
+    gp += gi * pi;
+    mx = fmax(mx, fabs(pi) / sqrt(fmax(a.xb[i >> 2].x, 1e-3)));
+    a.z0[i] = a.z[i];
+    a.g0[i] = gi;
+  }
+  gp = R.sum(gp);
+  double restart = 0.0;
+  if (!(gp < 0.0)) {  // not a descent direction: steepest descent
+    restart = 1.0;
+    used = 0;
+    gp = mx = 0.0;
+    for (int i = i0; i < n4; i += step) {
+      const double gi = a.g[i];
+      q[i] = -gi;
+      gp += gi * -gi;
+      mx = fmax(mx, fabs(gi) / sqrt(fmax(a.xb[i >> 2].x, 1e-3)));
+    }
+    gp = R.sum(gp);
+  }
+  // first step of a history: move no q (A) or log sigma by more than 0.05
+  const double pmax = R.max(mx);
+  if (rank == 0 && threadIdx.x == 0) {
+    a.out[0] = gp;
+    a.out[1] = used == 0 && pmax > 0.05 ? 0.05 / pmax : 1.0;
+    a.out[2] = restart;
+  }
+  R.end();
 }
 
 // Per-site scale of the optimisation variables: a site's energy terms carry
@@ -52,75 +255,111 @@ __device__ __forceinline__ double occ_scale(double x) { return sqrt(fmax(x, 1e-3
 // sigma components pinned at a bound with the gradient pointing outwards;
 // F = sum_active beta V0 - 3 sum_relaxed log sigma; the projected residual
 // |R|^2 over the relaxed sites.
-__global__ void gather_kernel(int n, const double4 *pos, const double2 *xb, const double *V0,
-                              const double *Rq, const double *Rs, RelaxBounds bd, double *z,
-                              double *g, double *fterm, double *rterm) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double4 p = pos[i];
-  double2 b = xb[i];
-  bool act = b.x >= 5e-4;
-  bool rel = act && b.x >= bd.x_min;
-  double sc = occ_scale(b.x), ls = log(p.w), be = b.y;
-  z[4 * i] = sc * p.x;
-  z[4 * i + 1] = sc * p.y;
-  z[4 * i + 2] = sc * p.z;
-  z[4 * i + 3] = sc * ls;
-  double gs = be * p.w * Rs[i];
-  bool pin = (ls >= bd.ls_hi - 1e-12 && gs < 0.0) || (ls <= bd.ls_lo + 1e-12 && gs > 0.0);
-  g[4 * i] = rel ? be * Rq[3 * i] / sc : 0.0;
-  g[4 * i + 1] = rel ? be * Rq[3 * i + 1] / sc : 0.0;
-  g[4 * i + 2] = rel ? be * Rq[3 * i + 2] / sc : 0.0;
-  g[4 * i + 3] = (rel && !pin) ? gs / sc : 0.0;
-  fterm[i] = act ? be * V0[i] - (rel ? 3.0 * ls : 0.0) : 0.0;
-  rterm[i] = rel ? Rq[3 * i] * Rq[3 * i] + Rq[3 * i + 1] * Rq[3 * i + 1] +
-                       Rq[3 * i + 2] * Rq[3 * i + 2] + (pin ? 0.0 : Rs[i] * Rs[i])
-                 : 0.0;
+// The two sums: a partial per block, the last block to finish adds the
+// partials in block order (fixed strides, fixed trees) and resets the count.
+constexpr int kGB = 128;
+__global__ void __launch_bounds__(kGB)
+gather_kernel(int n, const double4 *pos, const double2 *xb, const double *V0, const double *Rq,
+              const double *Rs, RelaxBounds bd, double *z, double *g, double *part,
+              unsigned *count, int *err, double *out) {
+  __shared__ double sh[2][kGB / 32];
+  __shared__ bool last;
+  double f = 0.0, r2 = 0.0;
+  for (int i = blockIdx.x * kGB + threadIdx.x; i < n; i += gridDim.x * kGB) {
+    double4 p = pos[i];
+    double2 b = xb[i];
+    bool act = b.x >= 5e-4;
+    bool rel = act && b.x >= bd.x_min;
+    double sc = occ_scale(b.x), ls = log(p.w), be = b.y;
+    z[4 * i] = sc * p.x;
+    z[4 * i + 1] = sc * p.y;
+    z[4 * i + 2] = sc * p.z;
+    z[4 * i + 3] = sc * ls;
+    double gs = be * p.w * Rs[i];
+    bool pin = (ls >= bd.ls_hi - 1e-12 && gs < 0.0) || (ls <= bd.ls_lo + 1e-12 && gs > 0.0);
+    g[4 * i] = rel ? be * Rq[3 * i] / sc : 0.0;
+    g[4 * i + 1] = rel ? be * Rq[3 * i + 1] / sc : 0.0;
+    g[4 * i + 2] = rel ? be * Rq[3 * i + 2] / sc : 0.0;
+    g[4 * i + 3] = (rel && !pin) ? gs / sc : 0.0;
+    f += act ? be * V0[i] - (rel ? 3.0 * ls : 0.0) : 0.0;
+    r2 += rel ? Rq[3 * i] * Rq[3 * i] + Rq[3 * i + 1] * Rq[3 * i + 1] +
+                    Rq[3 * i + 2] * Rq[3 * i + 2] + (pin ? 0.0 : Rs[i] * Rs[i])
+              : 0.0;
+  }
+  auto both = [&](double &a, double &b) {  // the block's sums, in thread 0
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      sh[0][threadIdx.x >> 5] = a;
+      sh[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      a = sh[0][0];
+      b = sh[1][0];
+      for (int w = 1; w < kGB / 32; ++w) {
+        a += sh[0][w];
+        b += sh[1][w];
+      }
+    }
+  };
+  both(f, r2);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = f;
+    part[2 * blockIdx.x + 1] = r2;
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  f = r2 = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kGB) {
+    f += __ldcg(part + 2 * b);
+    r2 += __ldcg(part + 2 * b + 1);
+  }
+  both(f, r2);
+  if (threadIdx.x == 0) {
+    out[0] = f;
+    out[1] = r2;
+    out[2] = (double)*err;  // the evaluation's error bits, read and cleared
+    *err = 0;
+    *count = 0;
+  }
 }
 
-// pos of real sites from w = w0 + alpha p (sigma = exp(s), s kept in bounds)
+// Rows of the real sites, then of their images, from w = w0 + alpha p (sigma =
+// exp(s), s kept in bounds); alpha = scale times *alpha_dev if given.  A site
+// below x_min is held: its position is left untouched.  An image takes its
+// owner's new position, formed again from the same operations, plus its shift.
 __global__ void apply_kernel(int n, const double2 *xb, const double *z0, const double *p,
-                             double alpha, RelaxBounds bd, double4 *pos) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+                             double scale, const double *alpha_dev, RelaxBounds bd, double4 *pos,
+                             RelaxImages im) {
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= n + im.n) return;
+  const double alpha = alpha_dev ? scale * *alpha_dev : scale;
+  const int i = row < n ? row : im.owner[row];
   const double x = xb[i].x;
-  if (!(x >= 5e-4 && x >= bd.x_min)) return;  // held fixed: position left untouched
+  if (!(x >= 5e-4 && x >= bd.x_min)) return;
   double sc = occ_scale(x);
-  double4 q = pos[i];
+  double4 q;
   q.x = (z0[4 * i] + alpha * p[4 * i]) / sc;
   q.y = (z0[4 * i + 1] + alpha * p[4 * i + 1]) / sc;
   q.z = (z0[4 * i + 2] + alpha * p[4 * i + 2]) / sc;
   double ls = (z0[4 * i + 3] + alpha * p[4 * i + 3]) / sc;
   q.w = exp(fmin(fmax(ls, bd.ls_lo), bd.ls_hi));
-  pos[i] = q;
-}
-
-__global__ void axpy_kernel(int n, const double *alpha, double sgn, const double *x, double *y) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] += sgn * (*alpha) * x[i];
-}
-__global__ void scale_kernel(int n, const double *num, const double *den, double *y) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    double d = *den;
-    y[i] *= (d > 0.0) ? (*num) / d : 1.0;
+  if (row >= n) {
+    const double qi[3] = {q.x, q.y, q.z};
+    double s[3];
+    image_position(im.box, im.image[row - n], qi, s);
+    q.x = s[0];
+    q.y = s[1];
+    q.z = s[2];
   }
-}
-__global__ void diff_kernel(int n, const double *a, const double *b, double *out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = a[i] - b[i];
-}
-__global__ void neg_kernel(int n, const double *a, double *out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = -a[i];
-}
-// alpha_k = rho_k * (s_k . q) ; scalar helpers on device
-__global__ void mul_kernel(const double *a, const double *b, double *out) {
-  if (threadIdx.x == 0) *out = (*a) * (*b);
-}
-// beta_k = rho_k * (y_k . r); coefficient alpha_k - beta_k
-__global__ void sub_scal_kernel(const double *a, const double *b, double *out) {
-  if (threadIdx.x == 0) *out = (*a) - (*b);
+  pos[row] = q;
 }
 
 inline int nb(long long n) { return (int)((n + 255) / 256); }
@@ -129,17 +368,18 @@ inline int nb(long long n) { return (int)((n + 255) / 256); }
 
 cudaError_t relax_gather(int n, const double4 *pos, const double2 *xb, const double *V0,
                          const double *Rq, const double *Rs, const RelaxBounds &bd, double *z,
-                         double *g, double *fterm, double *rterm, double *f_out,
-                         double *r2_out, const double *ones, cudaStream_t st) {
-  gather_kernel<<<nb(n), 256, 0, st>>>(n, pos, xb, V0, Rq, Rs, bd, z, g, fterm, rterm);
-  dot_kernel<<<1, kRB, 0, st>>>(n, fterm, ones, f_out);
-  dot_kernel<<<1, kRB, 0, st>>>(n, rterm, ones, r2_out);
+                         double *g, double *part, unsigned *count, int *err, double *out,
+                         cudaStream_t st) {
+  const int need = (n + kGB - 1) / kGB, blocks = need < kRelaxParts ? need : kRelaxParts;
+  gather_kernel<<<blocks, kGB, 0, st>>>(n, pos, xb, V0, Rq, Rs, bd, z, g, part, count, err, out);
   return cudaGetLastError();
 }
 
 cudaError_t relax_apply(int n, const double2 *xb, const double *z0, const double *p,
-                        double alpha, const RelaxBounds &bd, double4 *pos, cudaStream_t st) {
-  apply_kernel<<<nb(n), 256, 0, st>>>(n, xb, z0, p, alpha, bd, pos);
+                        double scale, const double *alpha_dev, const RelaxBounds &bd,
+                        double4 *pos, const RelaxImages &im, cudaStream_t st) {
+  apply_kernel<<<nb((long long)n + im.n), 256, 0, st>>>(n, xb, z0, p, scale, alpha_dev, bd, pos,
+                                                        im);
   return cudaGetLastError();
 }
 
@@ -158,46 +398,11 @@ cudaError_t vec_axpby(int n, double a, const double *x, double b, const double *
 }
 
 cudaError_t vec_dot(int n, const double *a, const double *b, double *out, cudaStream_t st) {
-  dot_kernel<<<1, kRB, 0, st>>>(n, a, b, out);
-  return cudaGetLastError();
+  return launch_cluster(dot_kernel, cluster_of(n), st, n, a, b, out);
 }
 
-// Two-loop recursion: p = -H g from the stored pairs (s_k, y_k), newest last
-// in `order`; all scalars stay on the device.
-cudaError_t lbfgs_direction(int n4, const double *g, double *const *S, double *const *Y,
-                            const double *rho, const int *order, int m_used, double *p,
-                            double *work_q, double *alpha, double *tmp, cudaStream_t st) {
-  cudaMemcpyAsync(work_q, g, n4 * sizeof(double), cudaMemcpyDeviceToDevice, st);
-  for (int t = m_used - 1; t >= 0; --t) {
-    int k = order[t];
-    dot_kernel<<<1, kRB, 0, st>>>(n4, S[k], work_q, tmp);
-    mul_kernel<<<1, 32, 0, st>>>(rho + k, tmp, alpha + k);
-    axpy_kernel<<<nb(n4), 256, 0, st>>>(n4, alpha + k, -1.0, Y[k], work_q);
-  }
-  if (m_used > 0) {
-    int k = order[m_used - 1];
-    // H0 = (s.y)/(y.y) I
-    dot_kernel<<<1, kRB, 0, st>>>(n4, S[k], Y[k], tmp);
-    dot_kernel<<<1, kRB, 0, st>>>(n4, Y[k], Y[k], tmp + 1);
-    scale_kernel<<<nb(n4), 256, 0, st>>>(n4, tmp, tmp + 1, work_q);
-  }
-  for (int t = 0; t < m_used; ++t) {
-    int k = order[t];
-    dot_kernel<<<1, kRB, 0, st>>>(n4, Y[k], work_q, tmp + 2);
-    mul_kernel<<<1, 32, 0, st>>>(rho + k, tmp + 2, tmp + 3);
-    sub_scal_kernel<<<1, 32, 0, st>>>(alpha + k, tmp + 3, tmp + 4);
-    axpy_kernel<<<nb(n4), 256, 0, st>>>(n4, tmp + 4, 1.0, S[k], work_q);
-  }
-  neg_kernel<<<nb(n4), 256, 0, st>>>(n4, work_q, p);
-  return cudaGetLastError();
-}
-
-cudaError_t lbfgs_push(int n4, const double *z_new, const double *z_old, const double *g_new,
-                       const double *g_old, double *S, double *Y, double *sy, cudaStream_t st) {
-  diff_kernel<<<nb(n4), 256, 0, st>>>(n4, z_new, z_old, S);
-  diff_kernel<<<nb(n4), 256, 0, st>>>(n4, g_new, g_old, Y);
-  dot_kernel<<<1, kRB, 0, st>>>(n4, Y, S, sy);
-  return cudaGetLastError();
+cudaError_t lbfgs_step(const LbfgsStep &a, cudaStream_t st) {
+  return launch_cluster(lbfgs_step_kernel, cluster_of(a.n4), st, a);
 }
 
 }  // namespace btam

@@ -106,15 +106,9 @@ __global__ void ghost_refresh_kernel(int n_real, int n_ghost, double4 *pos,
   if (k >= n_ghost) return;
   int g = n_real + k, o = owner[g];
   double4 q = pos[o];
-  char4 t = image[k];
-  int d[3] = {-(int)t.x, -(int)t.y, -(int)t.z};
-  double qi[3] = {q.x, q.y, q.z}, p[3];
-  for (int a = 0; a < 3; ++a) {
-    double s = qi[a];
-    for (int c = 0; c < 3; ++c)
-      if (d[c] != 0) s = __dadd_rn(s, (double)(-d[c]) * b.A[c][a]);
-    p[a] = s;
-  }
+  const double qi[3] = {q.x, q.y, q.z};
+  double p[3];
+  image_position(b, image[k], qi, p);
   pos[g] = make_double4(p[0], p[1], p[2], q.w);
   xb[g] = xb[o];
   code[g] = code[o];

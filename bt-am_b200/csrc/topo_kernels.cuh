@@ -28,6 +28,19 @@ struct GhostBox {
   int ortho;
 };
 
+// Position of the image of a site at q: q plus its shift, a lattice vector at a
+// time in the order of the image construction.
+__device__ __forceinline__ void image_position(const GhostBox &b, char4 t, const double (&q)[3],
+                                               double (&p)[3]) {
+  const int d[3] = {-(int)t.x, -(int)t.y, -(int)t.z};
+  for (int a = 0; a < 3; ++a) {
+    double s = q[a];
+    for (int c = 0; c < 3; ++c)
+      if (d[c] != 0) s = __dadd_rn(s, (double)(-d[c]) * b.A[c][a]);
+    p[a] = s;
+  }
+}
+
 struct CellGrid {
   double lo[3];
   double edge, inv_edge;
