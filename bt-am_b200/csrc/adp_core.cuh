@@ -586,10 +586,10 @@ template <class R> BTAM_HD V3<R> dual_J(const Dual<R> &D, const Geo<R> &g) {
 
 // B(f, f) = u^2 s^2 / 2 + w^2 s^4 / 3 at one geometry, and its gradient
 // [u u' s + u^2 + 2/3 w w' s^3 + 4/3 w^2 s^2] r.
-template <class R> BTAM_HD R bff(const Geo<R> &g) {
-  R s2 = g.s * g.s;
-  return (R)0.5 * g.u * g.u * s2 + (R)(1.0 / 3.0) * g.w * g.w * s2 * s2;
+template <class R> BTAM_HD R bff_s2(R s2, R u, R w) {
+  return (R)0.5 * u * u * s2 + (R)(1.0 / 3.0) * w * w * s2 * s2;
 }
+template <class R> BTAM_HD R bff(const Geo<R> &g) { return bff_s2(g.s * g.s, g.u, g.w); }
 template <class R> BTAM_HD R bff_grad_coef(const Geo<R> &g) {
   R s2 = g.s * g.s;
   return g.u * g.du * g.s + g.u * g.u +
@@ -597,10 +597,9 @@ template <class R> BTAM_HD R bff_grad_coef(const Geo<R> &g) {
 }
 
 // Dual of X f(r0) (one feature scaled by X).
-template <class R> BTAM_HD Dual<R> dual_feat(const Geo<R> &g, R X) {
+template <class R> BTAM_HD Dual<R> dual_feat_s2(const Geo<R> &g, R s2, R X) {
   Dual<R> D;
   R hu = (R)0.5 * X * g.u, hw = (R)0.5 * X * g.w;
-  R s2 = g.s * g.s;
   D.a[0] = hu * g.r.x; D.a[1] = hu * g.r.y; D.a[2] = hu * g.r.z;
   R t = (R)(1.0 / 6.0) * X * g.w * s2;
   D.d[0] = hw * g.r.x * g.r.x - t;
@@ -610,6 +609,9 @@ template <class R> BTAM_HD Dual<R> dual_feat(const Geo<R> &g, R X) {
   D.o[1] = hw * g.r.x * g.r.z;
   D.o[2] = hw * g.r.y * g.r.z;
   return D;
+}
+template <class R> BTAM_HD Dual<R> dual_feat(const Geo<R> &g, R X) {
+  return dual_feat_s2(g, g.s * g.s, X);
 }
 
 template <class R> BTAM_HD void feat_add(Feat<R> &F, const Geo<R> &g) {
@@ -833,6 +835,68 @@ template <class R> BTAM_HD void feat_acc(R *acc, int base, const Geo<R> &g, R X)
   acc[base + 6] += xw * (x * y);
   acc[base + 7] += xw * (x * z);
   acc[base + 8] += xw * (y * z);
+}
+
+// A feature point: the vector r of a geometry with u and w there.
+template <class R> BTAM_HD Geo<R> geo_of(const V3<R> &r, R u, R w) {
+  Geo<R> g;
+  g.r = r;
+  g.u = u;
+  g.w = w;
+  return g;
+}
+// Part I without the pair rule: g0 += X f(r0), hsum += X sum_{6} f,
+// cross += X^2 B(sum_6 f, f(r0)) over the neighbour-displaced points
+// r0 -+ amt_j e_k.  u0, w0: the splines at r0; axis(k, uw): u and w at r0 - amt_j
+// e_k, then at r0 + amt_j e_k.
+template <class R, class AX>
+BTAM_HD void pass1_points_part1(const V3<R> &r0, R amt_j, R X, R u0, R w0, const AX &axis,
+                                R *acc) {
+  Feat<R> f0{};
+  feat_add(f0, geo_of(r0, u0, w0));
+  Feat<R> hs{};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    R uw[4];
+    axis(k, uw);
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg)
+      feat_add(hs, geo_of(disp(r0, k, sg ? amt_j : -amt_j), uw[2 * sg], uw[2 * sg + 1]));
+  }
+  for (int c = 0; c < 3; ++c) {
+    acc[kP1G0 + c] += X * f0.a[c];
+    acc[kP1H + c] += X * hs.a[c];
+  }
+  for (int c = 0; c < 6; ++c) {
+    acc[kP1G0 + 3 + c] += X * f0.l[c];
+    acc[kP1H + 3 + c] += X * hs.l[c];
+  }
+  acc[kP1Cross] += X * X * bpair_r(hs, f0);
+}
+// Part II for one axis k: G(d) of r0 + amt_i e_k at acc[0..8] and of r0 - amt_i
+// e_k at acc[9..17]; returns the two points' B(f, f).
+template <class R>
+BTAM_HD R pass1_points_axis(const V3<R> &r0, R amt_i, R X, int k, const R (&uw)[4], R *acc) {
+  R ss = (R)0;
+#pragma unroll
+  for (int sg = 0; sg < 2; ++sg) {
+    const Geo<R> g = geo_of(disp(r0, k, sg ? -amt_i : amt_i), uw[2 * sg], uw[2 * sg + 1]);
+    feat_acc(acc, 9 * sg, g, X);
+    ss += bff_s2(dot3(g.r, g.r), g.u, g.w);
+  }
+  return ss;
+}
+// u and w at r0 + amt e_k, then at r0 - amt e_k, from the tables.
+template <class R, class TV>
+BTAM_HD void axis_uw(const TV &T, const V3<R> &r0, int k, R amt, int pk, R (&uw)[4]) {
+#pragma unroll
+  for (int sg = 0; sg < 2; ++sg) {
+    Geo<R> g;
+    R p;
+    geo_uw<R, false>(g, disp(r0, k, sg ? -amt : amt), T, pk, p);
+    uw[2 * sg] = g.u;
+    uw[2 * sg + 1] = g.w;
+  }
 }
 
 // Part I without the pair rule: g0 += X f(r0), hsum += X sum_{6} f,
@@ -1317,6 +1381,47 @@ BTAM_HD void pass2_pair_sym(const TV &T, const V3<R> &r0, R sig_u, R sig_j, R xu
   }
   ou.gx += omega_uj * cros_x;
   oj.gx += omega_ju * rcros_x;
+}
+
+// ---------------------------------------------------------------------------
+// dV0_u/dx_j of a directed pair (u, j) from u's moments alone: u's part of j's
+// occupancy gradient (over beta_u / beta_j).  It is rcros_x of pass2_pair_sym;
+// no moments of j enter, so a site can hand it to all its neighbours as soon
+// as its own sums are done.  rho, phi, bff: the pair rule's sums (rho of j's
+// species); uw0: u and w at r0; axis(set, k, uw): u and w at the two points of an
+// axis, set 0: r0 + 3 sigma_u e_k, then r0 - 3 sigma_u e_k; set 1: r0 - 3 sigma_j
+// e_k, then r0 + 3 sigma_j e_k.
+template <class R, class MU, class AX>
+BTAM_HD R push_x(const V3<R> &r0, R sig_u, R sig_j, R xu, R xj, const MU &mu, R rho, R phi,
+                 R bffs, const R (&uw0)[2], const AX &axis) {
+  const R X = xu * xj;
+  R pair = (R)kW6 * (mu.scalar(1) * rho + (R)0.5 * xu * phi + (R)2 * X * xu * bffs);
+  const Geo<R> gc = geo_of(r0, uw0[0], uw0[1]);
+  const Dual<R> Xf0 = dual_feat_s2(gc, dot3(r0, r0), X);
+  R sum = dual_f(mu.dual(kDualH), gc);
+  const R amt_u = sig_u * (R)kDelta9, amt_j = sig_j * (R)kDelta9;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    R uw[4];
+    axis(0, k, uw);
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg) {
+      const Geo<R> g = geo_of(disp(r0, k, sg ? -amt_u : amt_u), uw[2 * sg], uw[2 * sg + 1]);
+      sum += dual_f(mu.dual(kDualGd + 2 * k + sg), g) - X * bff_s2(dot3(g.r, g.r), g.u, g.w);
+    }
+  }
+  const Dual<R> D5 = dual_sub(mu.dual(kDualG0), Xf0);
+  const DualAx<R> x5 = dual_ax(dual_sub(D5, Xf0), r0);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    R uw[4];
+    axis(1, k, uw);
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg)
+      sum += dual_ax_f(x5, k, sg ? amt_j : -amt_j,
+                       geo_of(r0, uw[2 * sg], uw[2 * sg + 1]));
+  }
+  return pair + (R)2 * (R)kW9 * xu * sum;
 }
 
 // ---------------------------------------------------------------------------

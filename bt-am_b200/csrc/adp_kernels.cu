@@ -942,6 +942,232 @@ pass2u_site_kernel(const EvalArgs<R> a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// X-only evaluations at fixed positions and widths (the master equation's
+// steps): only the occupancies change between them, so every spline value of a
+// slot is looked up once (keep_slots_kernel) and each evaluation streams them
+// (kept_site_kernel) instead of gathering 13 + 13 records per slot and a
+// 75-value moment record per pair.
+
+// One warp per site, a lane per slot, occupied or not.
+template <class R, int W>
+__global__ void __launch_bounds__(W * 32) keep_slots_kernel(const EvalArgs<R> a) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const RadialView<R> &T = a.T;
+#pragma unroll 1
+  for (int i = blockIdx.x * W + warp; i < a.n_real; i += gridDim.x * W) {
+    const double4 qi = a.pos[i];
+    const int ci = a.code[i];
+    const R amt_i = (R)qi.w * (R)kDelta9;
+#pragma unroll 1
+    for (int p = a.offs[i] + lane; p < a.offs[i + 1]; p += 32) {
+      const NbSite<R> sj = nb_site(a, a.idx[p]);
+      const V3<R> r0 = pair_vec<R>(qi, sj);
+      const int pk = pair_kind(ci, sj.code), so = a.slot_own[p];
+      const R amt_j = sj.sigma * (R)kDelta9;
+      auto put = [&](int c, const R (&v)[4]) {
+        st_rec4(a.kept + 4 * ((size_t)c * a.n_slots + p), v);
+      };
+      R rec[4];
+      ld4(a.prec1 + (size_t)kPr1 * (so >> 1), rec);
+      Geo<R> g;
+      R pp;
+      geo_uw<R, false>(g, r0, T, pk, pp);
+      const R c0[4] = {r0.x, r0.y, r0.z, sj.sigma};
+      const R c1[4] = {(so & 1) ? rec[0] : rec[1], rec[2], rec[3], g.u};
+      const R c2[4] = {g.w, (R)0, (R)0, (R)0};
+      put(0, c0);
+      put(1, c1);
+      put(2, c2);
+#pragma unroll
+      for (int s = 0; s < 6; ++s) {
+        R uw[4];
+        axis_uw<R>(T, r0, s % 3, s < 3 ? amt_i : -amt_j, pk, uw);
+        put(3 + s, uw);
+      }
+    }
+  }
+}
+
+// A moment record in shared memory, in the plain order.
+template <class R> struct MomShared {
+  const R *m;
+  __device__ __forceinline__ R scalar(int c) const { return m[c]; }
+  __device__ __forceinline__ Dual<R> dual(int k) const {
+    R h[8];
+    cp8(m + 8 + 8 * k, h);
+    return dual_from(h, m[72 + k]);
+  }
+};
+
+// A group of 16 lanes per site over its slots: the pass-1 sums, energy and
+// moment record from the kept values, then u's part of each neighbour's
+// occupancy gradient (push_x) into the reverse slot's gx.  What bounds it is
+// the latency and L2-to-SM stream of the kept values, read twice.  38,040-site
+// nanowire (FP32C), per step, before (pass 1 and pass 2 of the undirected
+// kernels) and after: 482 -> 314 us; 2,916-site cell (FP64): 79 -> 33.
+template <class R, int W, int MB>
+__global__ void __launch_bounds__(W * 32, MB) kept_site_kernel(const EvalArgs<R> a) {
+  constexpr int G = 16, SPW = 2, kOcc = 144;  // slots whose occupancy is cached
+  __shared__ SiteSums ss[W * SPW];
+  __shared__ R mu_s[W * SPW][kMomStride];
+  __shared__ R occ_s[W * SPW][kOcc];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = lane / G, sl = lane % G, gbase = half * G;
+  R *occ_c = occ_s[warp * SPW + half];
+#pragma unroll 1
+  for (int wi = blockIdx.x * W + warp; wi * SPW < a.n_real; wi += gridDim.x * W) {
+    const int i = wi * SPW + half;
+    const bool live = i < a.n_real;
+    const double2 xbi = live ? a.xb[i] : make_double2(0.0, 1.0);
+    const bool act = live && !(xbi.x < kMinOcc);
+    const R xi = (R)xbi.x;
+    const R sig_i = act ? (R)a.pos[i].w : (R)0, amt_i = sig_i * (R)kDelta9;
+    const int ci = act ? a.code[i] : 0;
+    const int nb0 = live ? a.offs[i] : 0, nb1 = live ? a.offs[i + 1] : 0;
+    const int end = act ? nb1 : nb0;
+    double *site = reinterpret_cast<double *>(&ss[warp * SPW + half]);
+    R *mu = mu_s[warp * SPW + half];
+    auto look = [&](int p) -> R {  // occupancy of slot p's neighbour, -1: empty
+      const double x = a.xb[a.idx[p]].x;
+      return x < kMinOcc ? (R)-1 : (R)x;
+    };
+    auto occ = [&](int p) -> R { return p - nb0 < kOcc ? occ_c[p - nb0] : look(p); };
+    auto chunk = [&](int c, int p, R(&v)[4]) {
+      ld4(a.kept + 4 * ((size_t)c * a.n_slots + p), v);
+    };
+    {
+      R acc[kP1PartI], lo[kP1PartI];
+#pragma unroll
+      for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
+#pragma unroll 1
+      for (int p = nb0 + sl; p < end; p += G) {
+        R c0[4], c1[4], c2[4], nb[3][4];
+        chunk(0, p, c0);
+        chunk(1, p, c1);
+        chunk(2, p, c2);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) chunk(6 + k, p, nb[k]);
+        const R xj = look(p);
+        if (p - nb0 < kOcc) occ_c[p - nb0] = xj;
+        if (xj < (R)0) continue;
+        const R X = xi * xj;
+        acc[kP1Rho] += xj * c1[0];
+        acc[kP1Epair] += (R)0.5 * X * c1[1];
+        acc[kP1Ediag] += X * X * c1[2];
+        pass1_points_part1<R>(
+            mk3<R>(c0[0], c0[1], c0[2]), c0[3] * (R)kDelta9, X, c1[3], c2[0],
+            [&](int k, R(&uw)[4]) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) uw[c] = nb[k][c];
+            },
+            acc);
+      }
+      lane_tree<G>(acc, lo, lane);
+      const int v0 = tree_base<kP1PartI, G>(sl);
+#pragma unroll
+      for (int k = 0; k < kP1PartI / G; ++k)
+        if (act && v0 + k < kP1Gd && v0 + k != kP1Sself)
+          site[p1_site_slot(v0 + k)] = tree_total(acc[k], lo[k]);
+    }
+    if constexpr (sizeof(R) == 4) {
+      R acc[kP1PartII], lo[kP1PartII];
+#pragma unroll
+      for (int c = 0; c < kP1PartII; ++c) acc[c] = (R)0;
+#pragma unroll 1
+      for (int p = nb0 + sl; p < end; p += G) {
+        R c0[4], uw[3][4];
+        chunk(0, p, c0);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) chunk(3 + k, p, uw[k]);
+        const R xj = occ(p);
+        if (xj < (R)0) continue;
+        const R X = xi * xj;
+        R s = (R)0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          s += pass1_points_axis(mk3<R>(c0[0], c0[1], c0[2]), amt_i, X, k, uw[k],
+                                 acc + 1 + 18 * k);
+        acc[0] += X * X * s;
+      }
+      lane_tree<G>(acc, lo, lane);
+      const int t0 = tree_base<kP1PartII, G>(sl);
+#pragma unroll
+      for (int k = 0; k < kP1PartII / G; ++k)
+        if (act && t0 + k < 1 + 54)
+          site[p1_site_slot(p1_part2_value(t0 + k))] = tree_total(acc[k], lo[k]);
+    } else {
+      double sself = 0.0;
+#pragma unroll 1
+      for (int ax = 0; ax < 3; ++ax) {
+        R acc[kP1PartI], lo[kP1PartI];
+#pragma unroll
+        for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
+#pragma unroll 1
+        for (int p = nb0 + sl; p < end; p += G) {
+          R c0[4], uw[4];
+          chunk(0, p, c0);
+          chunk(3 + ax, p, uw);
+          const R xj = occ(p);
+          if (xj < (R)0) continue;
+          const R X = xi * xj;
+          acc[0] += X * X * pass1_points_axis(mk3<R>(c0[0], c0[1], c0[2]), amt_i, X, ax, uw,
+                                              acc + 1);
+        }
+        lane_tree<G>(acc, lo, lane);
+        const int t0 = tree_base<kP1PartI, G>(sl);
+#pragma unroll
+        for (int k = 0; k < kP1PartI / G; ++k) {
+          const int t = t0 + k;
+          if (t == 0) sself += tree_total(acc[k], lo[k]);
+          else if (act && t < 1 + 18)
+            site[p1_site_slot(p1_part2_value(1 + 18 * ax + (t - 1)))] =
+                tree_total(acc[k], lo[k]);
+        }
+      }
+      if (act && sl == 0) site[p1_site_slot(kP1Sself)] = sself;
+    }
+    __syncwarp();
+    double b = 0.0;
+    if (act && sl < 8) b = site_dual(ss[warp * SPW + half], sl, mu);
+    double bgd = 0.0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) bgd += __shfl_sync(0xffffffffu, b, gbase + 2 + d);
+    if (act && sl == 0) {
+      SiteResult res;
+      site_scalars(ss[warp * SPW + half], bgd, a.emb[ci], xbi.x, ci, xbi.y, a.gamma[i],
+                   a.pos[i].w, a.mass[ci], res, mu);
+      a.rho[i] = res.rho;
+      a.V0[i] = res.V0;
+      a.S0[i] = res.S0;
+      a.selfx[i] = res.selfx;
+      if (!(finite(res.V0) && finite(res.S0) && finite(res.selfx)))
+        atomicOr(a.err, 1 << kErrBitNonFinite);
+    }
+    if (live && !act && sl == 0) a.rho[i] = a.V0[i] = a.S0[i] = a.selfx[i] = 0.0;
+    __syncwarp();
+    const MomShared<R> m{mu};
+#pragma unroll 1
+    for (int p = nb0 + sl; p < nb1; p += G) {
+      const int r = a.rev[p];
+      R gx = (R)0;
+      const R xj = act ? occ(p) : (R)-1;
+      if (!(xj < (R)0)) {
+        R c0[4], c1[4], c2[4];
+        chunk(0, p, c0);
+        chunk(1, p, c1);
+        chunk(2, p, c2);
+        const R uw0[2] = {c1[3], c2[0]};
+        gx = push_x<R>(mk3<R>(c0[0], c0[1], c0[2]), sig_i, c0[3], xi, xj, m, c1[0], c1[1], c1[2],
+                       uw0, [&](int set, int k, R(&uw)[4]) { chunk(3 + 3 * set + k, p, uw); });
+        if (!a.same_beta) gx *= (R)(xbi.y / a.xb[a.idx[p]].y);
+      }
+      if (r >= 0) a.pgx[r] = gx;
+    }
+    __syncwarp();  // the warp's shared buffers are reused by its next sites
+  }
+}
+
 // Deterministic FP64 totals in two stages.  Stage 1: block (b, k) sums the
 // sites [lo + len b / P, lo + len (b + 1) / P) of system k (lo = seg[k],
 // len = seg[k + 1] - lo; one system [0, n) when seg is null) with fixed
@@ -1066,6 +1292,16 @@ template <class R, int W, int MB> void go2(const EvalArgs<R> &a, cudaStream_t st
   k<<<grid_of(k, a.n_real, W, pers), W * 32, 0, st>>>(a);
 }
 
+// The packed neighbour rows of the current state.
+template <class R> void launch_pack(const EvalArgs<R> &a, cudaStream_t st) {
+  if (a.s32 && a.n_all > 0)
+    pack_sites_kernel<<<nblocks(a.n_all, 256), 256, 0, st>>>(a.n_all, a.pos, a.xb, a.code,
+                                                             a.owner, a.s32, a.sb);
+  if (a.s64 && a.n_all > 0)
+    pack_sites64_kernel<<<nblocks(a.n_all, 256), 256, 0, st>>>(a.n_all, a.pos, a.xb, a.code,
+                                                               a.owner, a.s64);
+}
+
 template <class R>
 cudaError_t launch_pass1(const EvalArgs<R> &a, cudaStream_t st, int v, int v2, cudaEvent_t mid) {
   if (a.n_real <= 0) return cudaSuccess;
@@ -1073,12 +1309,22 @@ cudaError_t launch_pass1(const EvalArgs<R> &a, cudaStream_t st, int v, int v2, c
   // the pair-rule records are made (and then also used by pass 1) whenever
   // either pass runs undirected: the undirected pass 2 reads them
   const bool und = ((v | v2) & kUndirected) != 0 && has_undirected(a);
-  if (a.s32 && a.n_all > 0)
-    pack_sites_kernel<<<nblocks(a.n_all, 256), 256, 0, st>>>(a.n_all, a.pos, a.xb, a.code,
-                                                             a.owner, a.s32, a.sb);
-  if (a.s64 && a.n_all > 0)
-    pack_sites64_kernel<<<nblocks(a.n_all, 256), 256, 0, st>>>(a.n_all, a.pos, a.xb, a.code,
-                                                               a.owner, a.s64);
+  if (und && a.x_only && a.kept) {
+    if (!a.recs_ready) {
+      launch_pack(a, st);
+      const int g = nblocks(a.n_own, 128);
+      if (g > 0) pass1u_pair_kernel<R, 128><<<g, 128, 0, st>>>(a);
+      if (mid) cudaEventRecord(mid, st);
+      keep_slots_kernel<R, 4><<<nblocks(a.n_real, 4), 128, 0, st>>>(a);
+    } else if (mid) {
+      cudaEventRecord(mid, st);
+    }
+    constexpr int MB = sizeof(R) == 8 ? 3 : 5;
+    auto k = kept_site_kernel<R, 4, MB>;
+    k<<<grid_of(k, (a.n_real + 1) / 2, 4, true), 128, 0, st>>>(a);
+    return cudaGetLastError();
+  }
+  launch_pack(a, st);
   switch (v & (kPersistent - 1)) {
   case 1: go1<R, 4, 5, 8>(a, st, pers, und, mid); break;
   case 2: go1<R, 4, 4, 16>(a, st, pers, und, mid); break;
@@ -1130,6 +1376,12 @@ template <class R>
 cudaError_t launch_pass2(const EvalArgs<R> &a, cudaStream_t st, int v, cudaEvent_t mid) {
   if (a.n_real <= 0) return cudaSuccess;
   const bool pers = (v & kPersistent) != 0;
+  if ((v & kUndirected) && has_undirected(a) && a.x_only && a.kept) {
+    if (mid) cudaEventRecord(mid, st);
+    auto ks = pass2u_site_kernel<R, 4>;
+    ks<<<grid_of(ks, a.n_real, 4, true), 128, 0, st>>>(a);
+    return cudaGetLastError();
+  }
   if ((v & kUndirected) && has_undirected(a)) {
     switch (v & (kPersistent - 1)) {
     case 1: go2u<R, 128, 5>(a, st, pers, mid); break;

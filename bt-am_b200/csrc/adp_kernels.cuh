@@ -78,7 +78,19 @@ template <class R> struct EvalArgs {
   // (2 t + 0 owned slot, + 1 its reverse)
   R *prec1 = nullptr, *prec2 = nullptr;
   const int *slot_own = nullptr;
+  // Values of every slot of the real sites' lists that do not change while
+  // positions and widths do not, for x-only evaluations, kKeptChunks chunks of
+  // four per slot (chunk c of slot p at 4 (c n_slots + p), so that the lanes of
+  // a site read whole lines); nullptr: none.  recs_ready: they are there from
+  // an earlier launch, else pass 1 makes them.
+  R *kept = nullptr;
+  long long n_slots = 0;
+  int same_beta = 0;  // beta is the same at both ends of every pair
 };
+// Chunks: 0 r0 and sigma_j; 1 the pair rule's sums rho, phi, B(f, f), and u at r0;
+// 2 w at r0, 0, 0, 0; 3 + s u and w at the two points of axis s mod 3 of set s / 3,
+// in the order of push_x.
+constexpr int kKeptChunks = 9;
 
 // Pass 1: rho-bar, V0, S0, dV0/dx (self) and the moment record of every
 // real site.  Pass 2: residuals of every real site.  `variant` picks the

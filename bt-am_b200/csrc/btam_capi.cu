@@ -282,6 +282,7 @@ template <class R> EvalArgs<R> eval_args(btam_system *s, R *mom, const RadialVie
   a.n_own = s->n_own;
   a.pbuf = reinterpret_cast<R *>(s->pbuf);
   a.slot_own = s->slot_own;
+  a.same_beta = s->same_beta ? 1 : 0;
   if (s->pbuf) {
     a.pgx = a.pbuf + pbuf_gx_offset(s->n_pairs);
     a.prec1 = a.pbuf + pbuf_prec1_offset(s->n_pairs);
@@ -333,9 +334,10 @@ void release_state_slots(btam_system *s);
 // master-equation steps made them), so pass 1 skips that kernel.  A served
 // job's evaluation goes to the server's batcher in full.  totals: also the
 // system's totals (the solvers form their own sums and complete the totals
-// once, at the end).
+// once, at the end).  kept: slot values of an x-only run (EvalArgs::kept), made
+// by its first evaluation.
 static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_ready,
-                        bool totals = true) {
+                        bool totals = true, void *kept = nullptr) {
   if (!s) return BTAM_ERR_ARG;
   if (!s->built) return BTAM_ERR_NOT_BUILT;
   if (precision != BTAM_FP64 && precision != BTAM_FP32C) return BTAM_ERR_ARG;
@@ -348,6 +350,8 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
     EvalArgs<double> a = eval_args<double>(s, s->mom64, s->T->r64);
     a.x_only = x_only;
     a.recs_ready = x_only && recs_ready;
+    a.kept = static_cast<double *>(kept);
+    a.n_slots = s->n_pairs;
     BTAM_TRY(launch_pass1(a, s->st, v1, v2));
     BTAM_TRY(launch_pass2(a, s->st, v2));
   } else {
@@ -355,6 +359,8 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
     EvalArgs<float> a = eval_args<float>(s, s->mom32, s->T->r32);
     a.x_only = x_only;
     a.recs_ready = x_only && recs_ready;
+    a.kept = static_cast<float *>(kept);
+    a.n_slots = s->n_pairs;
     BTAM_TRY(launch_pass1(a, s->st, v1, v2));
     BTAM_TRY(launch_pass2(a, s->st, v2));
   }
@@ -670,6 +676,8 @@ int btam_system_create(const btam_tables *t, int n, const double *q, const doubl
     delete s;
     return st;
   }
+  s->same_beta = true;  // beta is set here and never changes
+  for (int i = 1; beta && i < n; ++i) s->same_beta = s->same_beta && beta[i] == beta[0];
   cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete s;
@@ -729,7 +737,7 @@ void btam_system_destroy(btam_system *s) {
   dfree(s->mom64, s->st); dfree(s->mom32, s->st); dfree(s->err, s->st);
   dfree(s->doffs, s->st); dfree(s->didx, s->st); dfree(s->X, s->st); dfree(s->X0, s->st); dfree(s->dtot, s->st); dfree(s->mu, s->st);
   dfree(s->dctl, s->st);
-  dfree(s->dact, s->st); dfree(s->ddeg, s->st); dfree(s->rv, s->st);
+  dfree(s->dact, s->st); dfree(s->dout, s->st); dfree(s->din, s->st); dfree(s->rv, s->st);
   dfree(s->rev, s->st); dfree(s->slot_own, s->st); dfree(s->own_off, s->st); dfree(s->own_p, s->st); dfree(s->own_u, s->st);
   dfree(s->pbuf, s->st);
   s->scratch.release(s->st);
@@ -837,13 +845,17 @@ int btam_neighbors_build(btam_system *s, int all_sites) {
     BTAM_TRY(dalloc(s->slot_own, s->st, total));
     s->rev_cap = total;
   }
+  if (n + 5 > s->cnt_cap) {
+    BTAM_TRY(dalloc(s->cnt, s->st, n + 5));
+    s->cnt_cap = n + 5;
+  }
   if (n + 1 > s->own_off_cap) {
     BTAM_TRY(dalloc(s->own_off, s->st, n + 1));
     s->own_off_cap = n + 1;
   }
   BTAM_TRY(launch_pair_links(n, s->offs, s->idx, s->owner, s->rev, s->slot_own, s->cnt,
-                             s->own_off, s->own_p, s->own_u, s->own_cap, &s->n_own, s->scratch,
-                             s->st));
+                             s->own_off, s->own_p, s->own_u, s->own_cap, &s->n_own, &s->n_unpaired,
+                             s->scratch, s->st));
   // a rebuilt list may be longer than the pair buffer: pinned undirected
   // variants need it, the defaults take it again at the next evaluation
   bool pinned = false;
@@ -2047,6 +2059,14 @@ int btam_relax_newton(btam_system *s, double tol, int max_newton, int max_cg,
   return BTAM_OK;
 }
 
+}  // extern "C"
+
+namespace {
+DmdArgs dmd_args(btam_system *s);
+}
+
+extern "C" {
+
 int btam_dmd_setup(btam_system *s) {
   if (!s) return BTAM_ERR_ARG;
   if (!s->built) return BTAM_ERR_NOT_BUILT;
@@ -2064,12 +2084,10 @@ int btam_dmd_setup(btam_system *s) {
   BTAM_TRY(cudaMemsetAsync(s->dctl, 0, 3 * sizeof(unsigned long long), s->st));
   BTAM_TRY(dalloc(s->mu, s->st, n));
   BTAM_TRY(dalloc(s->dact, s->st, n));
-  BTAM_TRY(dalloc(s->ddeg, s->st, n));
+  BTAM_TRY(dalloc(s->dout, s->st, n));
+  BTAM_TRY(dalloc(s->din, s->st, n));
   BTAM_TRY(dmd_init(n, s->xb, s->code, s->X, s->st));
-  BTAM_TRY(dmd_commit_all(n, s->code, s->X, s->xb, s->st));
-  if (s->n_ghost > 0)
-    BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
-                                  s->box, s->st));
+  BTAM_TRY(dmd_commit(dmd_args(s), s->st));
   BTAM_TRY(cudaStreamSynchronize(s->st));
   s->dmd_ready = true;
   return BTAM_OK;
@@ -2093,6 +2111,7 @@ int dmd_params(const double *params, DmdParams &prm) {
 DmdArgs dmd_args(btam_system *s) {
   DmdArgs a;
   a.n = s->n_real;
+  a.n_all = s->n_real + s->n_ghost;
   a.xb = s->xb;
   a.code = s->code;
   a.owner = s->owner;
@@ -2106,18 +2125,32 @@ DmdArgs dmd_args(btam_system *s) {
   a.X0 = s->X0;
   a.mu = s->mu;
   a.active = s->dact;
-  a.deg = s->ddeg;
+  a.out = s->dout;
+  a.in = s->din;
   a.ctl = s->dctl;
   return a;
 }
 
-// Images follow their owners' new occupancies.
-int dmd_refresh_images(btam_system *s) {
-  if (s->n_ghost > 0)
-    BTAM_TRY(launch_ghost_refresh(s->n_real, s->n_ghost, s->pos, s->xb, s->code, s->owner,
-                                  s->image, s->box, s->st));
-  return BTAM_OK;
-}
+// Room for the kept slot values of a run of x-only evaluations (EvalArgs::kept):
+// with undirected variants and a reverse for every entry, if the memory may be
+// taken; nullptr else (the evaluations then look everything up each time).
+// Taken from the pool for the call and given back at its end.
+struct KeptSlots {
+  btam_system *s;
+  char *p = nullptr;
+  KeptSlots(btam_system *sys, int precision, int nsteps) : s(sys) {
+    const int f = precision == BTAM_FP64 ? 0 : 1;
+    int v1 = 0, v2 = 0;
+    if (nsteps <= 0 || !s->built || s->batcher || s->n_unpaired > 0 || s->n_list != s->n_real) return;
+    pick_variants(s, f, &v1, &v2);
+    size_t bytes = 0, elem = 0;
+    const size_t each = f == 0 ? sizeof(double) : sizeof(float);
+    const size_t values = 4 * (size_t)kKeptChunks * (size_t)std::max(s->n_pairs, 1ll);
+    if (((v1 | v2) & kUndirected) && values * each <= s->kept_limit)
+      take_pbuf(p, bytes, elem, values, each, s->st);
+  }
+  ~KeptSlots() { dfree(p, s->st); }
+};
 
 int dmd_finish(btam_system *s, long long *total_quanta) {
   if (total_quanta) {
@@ -2140,13 +2173,17 @@ int btam_dmd_step(btam_system *s, int precision, int nsteps, const double *param
   if (dmd_params(params, prm) != BTAM_OK) return BTAM_ERR_ARG;
   BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
   const DmdArgs a = dmd_args(s);
+  const KeptSlots kept(s, precision, nsteps);
   for (int k = 0; k < nsteps; ++k) {
     // chemical potentials at the current x; positions and widths do not
-    // move during the steps, so the pair-rule sums of the first are kept
-    int st = enqueue_eval(s, precision, true, k > 0);
+    // move during the steps, so what depends on them alone is kept
+    int st = enqueue_eval(s, precision, true, k > 0, false, kept.p);
     if (st != BTAM_OK) return st;
     BTAM_TRY(dmd_step(a, prm, s->st));
-    if ((st = dmd_refresh_images(s)) != BTAM_OK) return st;
+  }
+  if (nsteps > 0) {
+    int st = relax_totals(s);
+    if (st != BTAM_OK) return st;
   }
   return dmd_finish(s, total_quanta);
 }
@@ -2163,16 +2200,17 @@ int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *p
   const long long max_sub = (long long)max_sub_d;
   BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
   const DmdArgs a = dmd_args(s);
+  const KeptSlots kept(s, precision, nsteps);
   unsigned long long clip0 = 0;
   BTAM_TRY(copy_sync(&clip0, s->dctl + 2, sizeof(clip0), cudaMemcpyDeviceToHost, s->st));
   long long subs = 0, split = 0;
   double worst = 0.0;
   bool recs = false;  // the pair-rule sums of this call's positions are made
   for (int k = 0; k < nsteps; ++k) {
-    int st = enqueue_eval(s, precision, true, recs);
+    int st = enqueue_eval(s, precision, true, recs, false, kept.p);
     if (st != BTAM_OK) return st;
     recs = true;
-    BTAM_TRY(dmd_prepare(a, s->st));
+    BTAM_TRY(dmd_prepare(a, prm, s->st));
     BTAM_TRY(dmd_control(a, prm, max_dx, s->st));
     unsigned long long bits[2] = {0, 0};
     BTAM_TRY(copy_sync(bits, s->dctl, sizeof(bits), cudaMemcpyDeviceToHost, s->st));
@@ -2186,16 +2224,16 @@ int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *p
     sub.dt = prm.dt / (double)m;
     for (long long j = 0; j < m; ++j) {
       if (j > 0) {  // fresh chemical potentials for every later sub-step
-        if ((st = enqueue_eval(s, precision, true, true)) != BTAM_OK) return st;
-        BTAM_TRY(dmd_prepare(a, s->st));
+        if ((st = enqueue_eval(s, precision, true, true, false, kept.p)) != BTAM_OK) return st;
+        BTAM_TRY(dmd_prepare(a, prm, s->st));
       }
       BTAM_TRY(dmd_apply(a, sub, s->st));
-      if ((st = dmd_refresh_images(s)) != BTAM_OK) return st;
     }
     subs += m;
     split += m > 1;
   }
-  int st = dmd_finish(s, total_quanta);
+  int st = nsteps > 0 ? relax_totals(s) : BTAM_OK;
+  if (st == BTAM_OK) st = dmd_finish(s, total_quanta);
   if (stats) {
     unsigned long long clip1 = 0;
     BTAM_TRY(copy_sync(&clip1, s->dctl + 2, sizeof(clip1), cudaMemcpyDeviceToHost, s->st));

@@ -83,7 +83,8 @@ struct btam_system {
   long long *X = nullptr, *X0 = nullptr, *dtot = nullptr;
   unsigned long long *dctl = nullptr;  // step-control maxima and clip count (DmdArgs::ctl)
   double *mu = nullptr;
-  int *dact = nullptr, *ddeg = nullptr;
+  int *dact = nullptr;
+  long long *dout = nullptr, *din = nullptr;  // edge rooms (DmdArgs::out, in)
   // relaxation work vectors
   int relax_m = 0;
   double *rv = nullptr;  // one block holding every relaxation vector
@@ -92,6 +93,10 @@ struct btam_system {
       *own_u = nullptr;
   long long rev_cap = 0, own_cap = 0;
   int own_off_cap = 0, n_own = 0;
+  int n_unpaired = 0;      // entries without a reverse (rev < 0)
+  bool same_beta = false;  // every site has the same beta
+  // most bytes a master-equation call may take for kept slot values
+  size_t kept_limit = (size_t)-1;
   char *pbuf = nullptr;
   size_t pbuf_bytes = 0, pbuf_elem = 0;  // bytes; bytes per value (0: none yet)
   // non-mean-field forms: site records, outputs and totals (point.cu)

@@ -47,6 +47,11 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// Device memory that admission counts per neighbour slot: the pair links (4 +
+// 4), an FP64 slot record, and half an owned pair's indices and FP64 pair-rule
+// record.
+constexpr double kSlotBytes = 4 + 4 + 8 * 8 + 0.5 * (4 + 4 + (btam::kPrRec + 8) * 8);
+
 struct Job {
   long long id = 0;
   btam_job_spec spec{};
@@ -314,6 +319,10 @@ void run_job(btam_server *srv, Job *job) {
   } else if (st == BTAM_OK && !sp.plain) {
     st = btam_set_variants(s, BTAM_FP32C, kServeVariant1[1], kServeVariant2[1]);
     if (st == BTAM_OK) st = btam_set_variants(s, BTAM_FP64, kServeVariant1[0], kServeVariant2[0]);
+    // kept slot values only within what admission counted for the job's lists
+    const size_t counted = (size_t)n * BTAM_MAXNEIGH * kSlotBytes;
+    const size_t used = (size_t)s->n_pairs * 8 + s->pbuf_bytes + (size_t)s->n_own * 8;
+    s->kept_limit = counted > used ? counted - used : 0;
   } else if (st == BTAM_OK) {  // the plain two-pass pair
     st = btam_set_variants(s, BTAM_FP32C, 0, 0);
     if (st == BTAM_OK) st = btam_set_variants(s, BTAM_FP64, 0, 0);
@@ -428,7 +437,7 @@ long long btam_estimate_bytes(int n, const double cell[9], const int periodic[3]
   // at most one per two slots: the pair and site indices and an FP64
   // pair-rule record); plus a fixed allowance for cells and library scratch
   const double per_all = 32 + 16 + 4 + 4 + 4 + 4 + 4;
-  const double per_slot = 4 + 4 + 8 * 8 + 0.5 * (4 + 4 + (btam::kPrRec + 8) * 8);
+  const double per_slot = kSlotBytes;
   const double per_real = 8 + 40 + 48 + 24 + btam::kMomStride * 8 + btam::kMomStride * 4 + 8 + 256 * 4 +
                           BTAM_MAXNEIGH * 4 + 16 + 16 + 4 + BTAM_MAX_CHEMICAL_NEIGHS * 4 +
                           (2 * 8 + 8) * 5 * 8 + BTAM_MAXNEIGH * per_slot;

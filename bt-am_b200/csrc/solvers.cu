@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <vector>
 
 #include "solvers.cuh"
@@ -425,40 +426,58 @@ __global__ void dmd_init_kernel(int n, const double2 *xb, const int *code, long 
 }
 
 // chemical potential and diffusive activity (local H mass >= 0.01,
-// Topology.cpp:202-364) of every real H site
+// Topology.cpp:202-364) of every real H site: one warp per site, its lanes over
+// the list (a thread per site walked some 110 entries in turn: 34 us for 38,040
+// sites, a warp 10.6).  Occupancies are multiples of 2^-50, so a mass below 8 is
+// exact in any order of the sum and the test against 0.01 does not depend on
+// it.
 __global__ void dmd_mu_kernel(int n, const double2 *xb, const int *code, const double *Rx,
                               const double *gamma, const int *moffs, const int *midx,
                               const long long *X, double *mu, int *active) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= n) return;
   if (code[i] != 1) {
-    active[i] = 0;
-    mu[i] = 0.0;
+    if (lane == 0) {
+      active[i] = 0;
+      mu[i] = 0.0;
+    }
     return;
   }
-  double x = (double)X[i] * kDmdQuantum, beta = xb[i].y;
-  double mass = x;
-  for (int p = moffs[i]; p < moffs[i + 1]; ++p) {
-    int j = midx[p];
-    if (code[j] == 1) mass += xb[j].x;
+  double x = (double)X[i] * kDmdQuantum;
+  double mass = lane == 0 ? x : 0.0;
+  // past the threshold nothing more is needed (the terms are not negative)
+  for (int base = moffs[i]; base < moffs[i + 1]; base += 32) {
+    const int p = base + lane;
+    if (p < moffs[i + 1]) {
+      const int j = midx[p];
+      if (code[j] == 1) mass += xb[j].x;
+    }
+    if (__any_sync(0xffffffffu, mass >= 0.01)) break;
   }
+  for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+  if (lane != 0) return;
   active[i] = mass >= 0.01 ? 1 : 0;
   if (x >= 5e-4) {
+    const double beta = xb[i].y;
     mu[i] = Rx[i] + (x < 0.9999 ? gamma[i] / beta : 0.0);
   } else {
     double xt = x > 1e-12 ? x : 1e-12;
-    mu[i] = -(3.0 / (2.0 * xt) + 1.0 / (1.0 - xt)) / beta;
+    mu[i] = -(3.0 / (2.0 * xt) + 1.0 / (1.0 - xt)) / xb[i].y;
   }
 }
 
+// Active degree of every site, and the room one of its edges has under the
+// degree split: out, what the site may give, and in, what it may take.
 __global__ void dmd_degree_kernel(int n, const int *doffs, const int *didx, const int *owner,
-                                  const int *active, int *deg) {
+                                  const int *active, const long long *X, long long xmax,
+                                  long long *out, long long *in) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || !active[i]) return;
   int d = 0;
-  if (active[i])
-    for (int p = doffs[i]; p < doffs[i + 1]; ++p) d += active[owner[didx[p]]];
-  deg[i] = d;
+  for (int p = doffs[i]; p < doffs[i + 1]; ++p) d += active[owner[didx[p]]];
+  const long long di = d > 0 ? d : 1, x = X[i];
+  out[i] = x / di;
+  in[i] = xmax > x ? (xmax - x) / di : 0;
 }
 
 // Occupancy moved from i to o across an active edge in one step: dt J with
@@ -481,25 +500,21 @@ __device__ __forceinline__ long long dmd_quanta(double dlt) {
   return llrint(fmin(fmax(dlt * kDmdInvQuantum, -4e18), 4e18));
 }
 
-// The room of edge (i, o) in quanta under the degree split: a move from i
-// to o of at most hi, from o to i of at most -lo (lo <= 0).
-__device__ __forceinline__ void dmd_room(const long long *X, const int *deg, int i, int o,
-                                         long long xmax, long long &hi, long long &lo) {
-  const long long di = deg[i] > 0 ? deg[i] : 1, dq = deg[o] > 0 ? deg[o] : 1;
-  const long long out_i = X[i] / di, out_o = X[o] / dq;
-  const long long in_i = xmax > X[i] ? (xmax - X[i]) / di : 0;
-  const long long in_o = xmax > X[o] ? (xmax - X[o]) / dq : 0;
+// The room of edge (i, o) in quanta: a move from i to o of at most hi, from o
+// to i of at most -lo (lo <= 0).
+__device__ __forceinline__ void dmd_room(const long long *out, const long long *in, int i, int o,
+                                         long long &hi, long long &lo) {
+  const long long out_i = out[i], out_o = out[o], in_i = in[i], in_o = in[o];
   hi = out_i < in_o ? out_i : in_o;
   lo = -(out_o < in_i ? out_o : in_i);
 }
 
 __global__ void dmd_flux_kernel(int n, const double2 *xb, const int *doffs, const int *didx,
-                                const int *owner, const int *active, const int *deg,
-                                const double *mu, const long long *X0, long long *X,
-                                DmdParams prm, unsigned long long *ctl) {
+                                const int *owner, const int *active, const long long *out,
+                                const long long *in, const double *mu, const long long *X0,
+                                long long *X, DmdParams prm, unsigned long long *ctl) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || !active[i]) return;
-  const long long xmax = llrint(prm.max_x * kDmdInvQuantum);
   for (int p = doffs[i]; p < doffs[i + 1]; ++p) {
     int o = owner[didx[p]];
     if (o <= i || !active[o]) continue;  // each undirected edge once, from its lower end
@@ -507,7 +522,7 @@ __global__ void dmd_flux_kernel(int n, const double2 *xb, const int *doffs, cons
     if (fabs(dlt) < prm.min_dx) continue;
     long long q = dmd_quanta(dlt);
     long long hi, lo;
-    dmd_room(X0, deg, i, o, xmax, hi, lo);
+    dmd_room(out, in, i, o, hi, lo);
     // a move cut to a nonzero room is counted; a zero room (empty giver,
     // full receiver) moves nothing and is not
     if (ctl && ((q > hi && hi > 0) || (q < lo && lo < 0))) atomicAdd(ctl + 2, 1ull);
@@ -524,13 +539,12 @@ __global__ void dmd_flux_kernel(int n, const double2 *xb, const int *doffs, cons
 // nonzero room; the maxima go to ctl[1] and ctl[0] (a non-negative
 // double's bits order as the double).
 __global__ void dmd_control_kernel(int n, const double2 *xb, const int *doffs, const int *didx,
-                                   const int *owner, const int *active, const int *deg,
-                                   const double *mu, const long long *X, DmdParams prm,
-                                   double max_dx, unsigned long long *ctl) {
+                                   const int *owner, const int *active, const long long *out,
+                                   const long long *in, const double *mu, const long long *X,
+                                   DmdParams prm, double max_dx, unsigned long long *ctl) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double ratio = 0.0, dx = 0.0;
   if (i < n && active[i]) {
-    const long long xmax = llrint(prm.max_x * kDmdInvQuantum);
     for (int p = doffs[i]; p < doffs[i + 1]; ++p) {
       int o = owner[didx[p]];
       if (o == i || !active[o]) continue;
@@ -540,7 +554,7 @@ __global__ void dmd_control_kernel(int n, const double2 *xb, const int *doffs, c
       if (o < i) continue;  // the room of each edge once
       const long long q = dmd_quanta(dlt);
       long long hi, lo;
-      dmd_room(X, deg, i, o, xmax, hi, lo);
+      dmd_room(out, in, i, o, hi, lo);
       if (q > hi && hi > 0) ratio = fmax(ratio, (double)q / (double)hi);
       if (q < lo && lo < 0) ratio = fmax(ratio, (double)q / (double)lo);
     }
@@ -557,10 +571,15 @@ __global__ void dmd_control_kernel(int n, const double2 *xb, const int *doffs, c
   }
 }
 
-__global__ void dmd_commit_kernel(int n, const int *code, const long long *X, double2 *xb) {
+// x of every H row (real sites, then images) from its owner's quanta; the
+// quanta themselves become the next step's snapshot.
+__global__ void dmd_commit_kernel(int n, int n_all, const int *code, const int *owner,
+                                  const long long *X, long long *X0, double2 *xb) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || code[i] != 1) return;
-  xb[i].x = (double)X[i] * kDmdQuantum;
+  if (i >= n_all) return;
+  const long long q = X[i < n ? i : owner[i]];
+  if (i < n) X0[i] = q;
+  if (code[i] == 1) xb[i].x = (double)q * kDmdQuantum;
 }
 
 // exact total of the quanta (128-bit), single block, fixed order
@@ -592,16 +611,17 @@ cudaError_t dmd_init(int n, const double2 *xb, const int *code, long long *X, cu
   return cudaGetLastError();
 }
 
-cudaError_t dmd_commit_all(int n, const int *code, const long long *X, double2 *xb,
-                           cudaStream_t st) {
-  dmd_commit_kernel<<<nbk(n), 256, 0, st>>>(n, code, X, xb);
+cudaError_t dmd_commit(const DmdArgs &a, cudaStream_t st) {
+  dmd_commit_kernel<<<nbk(a.n_all), 256, 0, st>>>(a.n, a.n_all, a.code, a.owner, a.X, a.X0, a.xb);
   return cudaGetLastError();
 }
 
-cudaError_t dmd_prepare(const DmdArgs &a, cudaStream_t st) {
-  dmd_mu_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.xb, a.code, a.Rx, a.gamma, a.moffs, a.midx,
-                                          a.X, a.mu, a.active);
-  dmd_degree_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.doffs, a.didx, a.owner, a.active, a.deg);
+cudaError_t dmd_prepare(const DmdArgs &a, const DmdParams &prm, cudaStream_t st) {
+  dmd_mu_kernel<<<nbk((long long)a.n * 32), 256, 0, st>>>(a.n, a.xb, a.code, a.Rx, a.gamma,
+                                                          a.moffs, a.midx, a.X, a.mu, a.active);
+  dmd_degree_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.doffs, a.didx, a.owner, a.active, a.X,
+                                              std::llrint(prm.max_x * kDmdInvQuantum), a.out,
+                                              a.in);
   return cudaGetLastError();
 }
 
@@ -610,22 +630,18 @@ cudaError_t dmd_control(const DmdArgs &a, const DmdParams &prm, double max_dx,
   cudaError_t e = cudaMemsetAsync(a.ctl, 0, 2 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   dmd_control_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.xb, a.doffs, a.didx, a.owner, a.active,
-                                               a.deg, a.mu, a.X, prm, max_dx, a.ctl);
+                                               a.out, a.in, a.mu, a.X, prm, max_dx, a.ctl);
   return cudaGetLastError();
 }
 
 cudaError_t dmd_apply(const DmdArgs &a, const DmdParams &prm, cudaStream_t st) {
-  cudaError_t e = cudaMemcpyAsync(a.X0, a.X, (size_t)a.n * sizeof(long long),
-                                  cudaMemcpyDeviceToDevice, st);
-  if (e != cudaSuccess) return e;
   dmd_flux_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.xb, a.doffs, a.didx, a.owner, a.active,
-                                            a.deg, a.mu, a.X0, a.X, prm, a.ctl);
-  dmd_commit_kernel<<<nbk(a.n), 256, 0, st>>>(a.n, a.code, a.X, a.xb);
-  return cudaGetLastError();
+                                            a.out, a.in, a.mu, a.X0, a.X, prm, a.ctl);
+  return dmd_commit(a, st);
 }
 
 cudaError_t dmd_step(const DmdArgs &a, const DmdParams &prm, cudaStream_t st) {
-  cudaError_t e = dmd_prepare(a, st);
+  cudaError_t e = dmd_prepare(a, prm, st);
   return e == cudaSuccess ? dmd_apply(a, prm, st) : e;
 }
 

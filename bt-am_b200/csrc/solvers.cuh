@@ -70,15 +70,16 @@ struct DmdParams {
 };
 
 struct DmdArgs {
-  int n;  // real sites
+  int n, n_all;  // real sites; with their images
   double2 *xb;
   const int *code, *owner;
   const double *Rx, *gamma;
   const int *moffs, *midx;  // mechanical neighbours (real sites)
   const int *doffs, *didx;  // diffusive neighbours (real sites)
-  long long *X, *X0;        // occupancy quanta, snapshot
+  long long *X, *X0;        // occupancy quanta, snapshot at the step's start
+  long long *out, *in;      // quanta an edge of the site may give, take
   double *mu;
-  int *active, *deg;
+  int *active;
   // step-control counters: [0] the largest edge move over its room and [1]
   // the largest site change over max_dx of the last decision (non-negative
   // doubles as their bits), [2] edge moves clipped to a nonzero room
@@ -86,15 +87,14 @@ struct DmdArgs {
 };
 
 cudaError_t dmd_init(int n, const double2 *xb, const int *code, long long *X, cudaStream_t st);
-// x of every real H site from its quanta
-cudaError_t dmd_commit_all(int n, const int *code, const long long *X, double2 *xb,
-                           cudaStream_t st);
+// x of every H site and image from the quanta, which become the snapshot.
+cudaError_t dmd_commit(const DmdArgs &a, cudaStream_t st);
 cudaError_t dmd_step(const DmdArgs &a, const DmdParams &prm, cudaStream_t st);
-// The step in its parts: chemical potentials, activity and degrees of the
+// The step in its parts: chemical potentials, activity and rooms of the
 // current state; then (optionally) the step-control decision for a step
 // of prm.dt into ctl[0..1]; then the occupancy update of one step of
-// prm.dt (snapshot, edge moves, commit).
-cudaError_t dmd_prepare(const DmdArgs &a, cudaStream_t st);
+// prm.dt (edge moves, commit).
+cudaError_t dmd_prepare(const DmdArgs &a, const DmdParams &prm, cudaStream_t st);
 cudaError_t dmd_control(const DmdArgs &a, const DmdParams &prm, double max_dx, cudaStream_t st);
 cudaError_t dmd_apply(const DmdArgs &a, const DmdParams &prm, cudaStream_t st);
 cudaError_t dmd_total(int n, const int *code, const long long *X, long long *out2,

@@ -375,6 +375,8 @@ __device__ int reverse_slot(int u, bool real_pair, int o, int n_real, const int 
   return -1;
 }
 
+// own_cnt: owned entries of each site; entries without a reverse at n_real + 1
+// (zero before).
 __global__ void pair_rev_kernel(int n_real, const int *offs, const int *idx, const int *owner,
                                 int *rev, int *own_cnt) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -387,11 +389,21 @@ __global__ void pair_rev_kernel(int n_real, const int *offs, const int *idx, con
       int j = idx[p], o = owner[j];
       int r = reverse_slot(u, j < n_real, o, n_real, offs, idx, owner);
       rev[p] = r;
+      if (r < 0) atomicAdd(own_cnt + n_real + 1, 1);
       own = (u < o) || r < 0;
     }
     cnt += __popc(__ballot_sync(0xffffffffu, own));
   }
   if (lane == 0) own_cnt[u] = cnt;
+}
+
+// out: owned pairs, slots of the real sites' lists, entries without a reverse.
+__global__ void pair_totals_kernel(int n_real, const int *own_off, const int *own_cnt,
+                                   const int *offs, int *out) {
+  const int unpaired = own_cnt[n_real + 1];
+  out[0] = own_off[n_real];
+  out[1] = offs[n_real];
+  out[2] = unpaired;
 }
 
 // Owned pairs in site order, and every slot's owned pair and direction:
@@ -420,20 +432,23 @@ __global__ void pair_own_kernel(int n_real, const int *offs, const int *idx, con
 
 cudaError_t launch_pair_links(int n_real, const int *offs, const int *idx, const int *owner,
                               int *rev, int *slot_own, int *own_cnt, int *own_off, int *&own_p,
-                              int *&own_u, long long &own_cap, int *n_own,
+                              int *&own_u, long long &own_cap, int *n_own, int *n_unpaired,
                               DeviceScratch &scratch, cudaStream_t st) {
   cudaError_t e;
-  *n_own = 0;
+  *n_own = *n_unpaired = 0;
   if (n_real <= 0) return cudaSuccess;
   const int blocks = (int)(((long long)n_real * 32 + 127) / 128);
+  if ((e = cudaMemsetAsync(own_cnt + n_real, 0, 2 * sizeof(int), st)) != cudaSuccess) return e;
   pair_rev_kernel<<<blocks, 128, 0, st>>>(n_real, offs, idx, owner, rev, own_cnt);
-  if ((e = cudaMemsetAsync(own_cnt + n_real, 0, sizeof(int), st)) != cudaSuccess) return e;
   if ((e = exclusive_scan(own_cnt, own_off, n_real + 1, scratch, st)) != cudaSuccess) return e;
-  int total = 0;
-  if ((e = cudaMemcpyAsync(&total, own_off + n_real, sizeof(int), cudaMemcpyDeviceToHost, st)) !=
+  // the three counts in one copy
+  int tot[3];
+  pair_totals_kernel<<<1, 1, 0, st>>>(n_real, own_off, own_cnt, offs, own_cnt + n_real + 2);
+  if ((e = cudaMemcpyAsync(tot, own_cnt + n_real + 2, sizeof(tot), cudaMemcpyDeviceToHost, st)) !=
       cudaSuccess)
     return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  const int total = tot[0], n_slots = tot[1];
   if (total > own_cap) {
     cudaMemPool_t pool = device_pool();
     if (!pool) return cudaErrorMemoryAllocation;
@@ -449,17 +464,13 @@ cudaError_t launch_pair_links(int n_real, const int *offs, const int *idx, const
       return e;
     own_cap = total;
   }
-  int n_slots = 0;
-  if ((e = cudaMemcpyAsync(&n_slots, offs + n_real, sizeof(int), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
-    return e;
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   if (n_slots > 0 &&
       (e = cudaMemsetAsync(slot_own, 0xff, (size_t)n_slots * sizeof(int), st)) != cudaSuccess)
     return e;
   pair_own_kernel<<<blocks, 128, 0, st>>>(n_real, offs, idx, owner, rev, own_off, own_p, own_u,
                                           slot_own);
   *n_own = total;
+  *n_unpaired = tot[2];
   return cudaGetLastError();
 }
 

@@ -111,11 +111,11 @@ cudaError_t launch_neighbors(const NbrArgs &a, cudaStream_t st);
 // owner of idx[p], or -1 if o's list lacks it (rounding at exactly rc for an
 // image pair); slot p is owned by its site u when u < o or rev[p] < 0, and the
 // owned slots are listed as (own_p, own_u) in site-then-slot order.
-// own_cnt / own_off: n_real + 1 ints of scratch; *n_own returned after a
-// stream synchronisation.
+// own_cnt: n_real + 5 ints of scratch, own_off: n_real + 1; *n_own and
+// *n_unpaired (entries with rev < 0) returned after a stream synchronisation.
 cudaError_t launch_pair_links(int n_real, const int *offs, const int *idx, const int *owner,
                               int *rev, int *slot_own, int *own_cnt, int *own_off, int *&own_p,
-                              int *&own_u, long long &own_cap, int *n_own,
+                              int *&own_u, long long &own_cap, int *n_own, int *n_unpaired,
                               DeviceScratch &scratch, cudaStream_t st);
 
 cudaError_t launch_compact(int n_query, const int *tmp, const int *offs, int *idx,

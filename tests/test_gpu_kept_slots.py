@@ -1,0 +1,81 @@
+"""Master-equation steps on kept slot values (kept_site_kernel) against the
+general x-only evaluation of the same state.
+
+Forms: periodic and open, with empty sites, sites whose lists differ in length
+down to a few entries, one beta and many, both arithmetic forms.  The kept
+path forms the same terms from the same spline values; sums of a list of up to
+250 terms differ in order and contraction, so the chemical potentials agree to
+1e-13 (FP64) and 1e-6 (FP32C) of max(1, the largest), the tolerances of the
+x-only test.  Lists that cover the images do not take the kept path: there the
+two must agree to the same tolerance as well."""
+import numpy as np
+import pytest
+
+import btam
+from btam import lattice
+
+pytestmark = pytest.mark.gpu
+
+TOL = {btam.FP64: 1e-13, btam.FP32C: 1e-6}
+PRM = dict(dt=1e-3, Df=0.045, dr=3.2, min_dx=1e-8, max_x=0.9)
+
+
+def emptied(s, every=6):
+    x = s["x"].copy()
+    h = np.flatnonzero(s["species"] == 1)[::every]
+    x[h] = np.where(np.arange(len(h)) % 2 == 0, 1e-4, 0.0)
+    return dict(s, x=x)
+
+
+def many_betas(s):
+    g = np.random.default_rng(3)
+    n = len(s["x"])
+    return dict(s, beta=s["beta"] * g.uniform(0.8, 1.2, n), gamma=g.uniform(-0.5, 0.5, n))
+
+
+def cell():
+    return emptied(lattice.supercell(5, 5, 5, h_fraction=0.6, x_range=(0.0, 0.6),
+                                     sigma_range=(0.08, 0.15), jitter=0.02, seed=21))
+
+
+SYSTEMS = {
+    "cell": cell,
+    "cell_many_betas": lambda: many_betas(cell()),
+    "small_sphere": lambda: emptied(lattice.cluster(
+        "sphere", 5.0, x_fn=lambda g, r, n: g.uniform(0.0, 0.5, n), h_fraction=0.5, seed=22)),
+    "wire": lambda: lattice.wire(9.0, 5, seed=23),
+}
+
+
+@pytest.mark.parametrize("prec", [btam.FP64, btam.FP32C])
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_kept_potentials_equal_the_general_ones(gpu_tables, name, prec):
+    s = SYSTEMS[name]()
+    A = btam.System(gpu_tables, s)
+    A.build_neighbors()
+    A.set_variants(prec, 16 | 2, 16 | 1)
+    A.dmd_setup()
+    B = btam.System(gpu_tables, s)
+    B.build_neighbors(all_sites=True)
+    B.set_variants(prec, 16 | 2, 16 | 1)
+    B.dmd_setup()
+    for step in range(3):
+        x, _, _ = A.dmd_occupancy()
+        A.set_state(x=x)
+        ref = A.evaluate_x(prec)  # the general x-only evaluation of this state
+        B.set_state(x=x)
+        ta, tb = A.dmd_step(1, prec, **PRM), B.dmd_step(1, prec, **PRM)
+        assert ta == tb
+        got = A.results(want=("rho", "V0", "Rx", "Rq", "Rs"))
+        assert not np.any(got["Rq"]) and not np.any(got["Rs"])
+        for k in ("rho", "V0", "Rx"):
+            d = np.abs(got[k] - ref[k]).max()
+            print(name, prec, step, k, d)
+            assert d <= TOL[prec] * max(1.0, np.abs(ref[k]).max()), (name, k, step, d)
+        xa, _, mu = A.dmd_occupancy()
+        h = (s["species"] == 1) & (x >= 5e-4)
+        want = ref["Rx"] + np.where(x < 0.9999, s["gamma"] / s["beta"], 0.0)
+        assert np.abs(mu - want)[h].max() <= TOL[prec] * max(1.0, np.abs(want[h]).max())
+        xb, Xb, _ = B.dmd_occupancy()
+        # a potential's last bits move at most a few quanta's worth of x
+        assert np.abs(xa - xb).max() <= 10 * TOL[prec]
