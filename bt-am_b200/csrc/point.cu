@@ -23,6 +23,7 @@
 //           dV_u/dq_a (x) q0_a.
 // A lane per neighbour, a warp per site, fixed-order warp reductions: the
 // results are deterministic.
+#include <algorithm>
 #include <cmath>
 #include <functional>
 #include <cstring>
@@ -227,6 +228,150 @@ __global__ void __launch_bounds__(128) pt_grad_kernel(PtArgs a, double *slot3) {
   if (lane == 0) {
     for (int c = 0; c < 3; ++c) a.Fq[3 * (size_t)u + c] = acc[c];
     for (int c = 0; c < 9; ++c) a.W[9 * (size_t)u + c] = acc[3 + c];
+  }
+}
+
+// Diagonal of the total stress, sum_u W_u(a, a), at the stretched positions
+// diag(F) q: the residual of the bulk stretch relaxation, which needs nothing
+// else of the point forms.  W_u depends on u's own list and moments alone, so
+// one warp per site does both: each lane looks its entries' splines up once,
+// the warp sums rho, mu and Lambda, and the lanes add g(u->j)_a r_a of the
+// entries, which they still hold (kPtHold a lane; the entries of a longer list
+// are looked up a second time).  A lane carries its three sums over all its
+// sites; the last block adds the blocks' partials in their order and hands the
+// error bits over with the sums.  Against the two passes over the lists, the
+// per-site outputs and their totals (81 + 156 + 11 us for 27,000 sites, and 4
+// for moving the sites and images first) it takes 125 us.  The lookups' L1
+// traffic and latency bound it: 4 entries a lane hold the usual list (up to 128)
+// in 164 registers, three blocks of 4 warps an SM.  5 entries at two blocks took
+// 156 us; 2 entries at four blocks (lists over 64 looked up twice) 127.
+constexpr int kPtHold = 4;
+struct PtEntry {
+  V3<double> r;
+  double A, B;    // x_j rho'/s, t phi' / (2 s)
+  double tu, tdu; // t u, t u'/s
+  double tw, tdw; // t w, t w'/s
+  double rho;     // x_j rho
+};
+__device__ __forceinline__ PtEntry pt_entry(const PtArgs &a, const V3<double> &F, int p, int end,
+                                            const double4 &qi, int ci, double xi) {
+  PtEntry e;
+  e.r = mk3<double>(0.0, 0.0, 0.0);
+  e.A = e.B = e.tu = e.tdu = e.tw = e.tdw = e.rho = 0.0;
+  if (p >= end) return e;
+  const int j = a.idx[p];
+  const double xj = a.xb[j].x;
+  if (xj < kMinOcc) return e;
+  const double4 qj = a.pos[j];
+  const int cj = a.code[j], pk = pair_kind(ci, cj);
+  e.r = mk3<double>(F.x * (qj.x - qi.x), F.y * (qj.y - qi.y), F.z * (qj.z - qi.z));
+  Geo<double> g;
+  double pp, ph, dph, rj, drj, ri, dri;
+  const int m = geo_uw<double, true>(g, e.r, a.T, pk, pp);
+  pr_at<double, true, false>(a.T, pk, ci, cj, m, pp, ph, dph, rj, drj, ri, dri);
+  const double t = xi * xj;
+  e.A = xj * drj * g.inv_s;
+  e.B = 0.5 * (t * dph) * g.inv_s;
+  e.tu = t * g.u;
+  e.tdu = t * g.du * g.inv_s;
+  e.tw = t * g.w;
+  e.tdw = t * g.dw * g.inv_s;
+  e.rho = xj * rj;
+  return e;
+}
+__device__ __forceinline__ void pt_entry_sums(const PtEntry &e, double (&m)[10]) {
+  m[0] += e.rho;
+  m[1] += e.tu * e.r.x;
+  m[2] += e.tu * e.r.y;
+  m[3] += e.tu * e.r.z;
+  const double wx = e.tw * e.r.x, wy = e.tw * e.r.y;
+  m[4] += wx * e.r.x;
+  m[5] += wy * e.r.y;
+  m[6] += e.tw * e.r.z * e.r.z;
+  m[7] += wy * e.r.z;
+  m[8] += wx * e.r.z;
+  m[9] += wx * e.r.y;
+}
+// g(u->j)_a r_a of an entry, from u's sums (m: as pt_entry_sums, m[0] = x F').
+__device__ __forceinline__ void pt_entry_stress(const PtEntry &e, const double (&m)[10],
+                                                double tr, double (&w)[3]) {
+  const V3<double> &r = e.r;
+  const V3<double> Lr = mk3<double>(m[4] * r.x + m[9] * r.y + m[8] * r.z,
+                                    m[9] * r.x + m[5] * r.y + m[7] * r.z,
+                                    m[8] * r.x + m[7] * r.y + m[6] * r.z);
+  const double s2 = dot3(r, r);
+  const double k = m[0] * e.A + e.B + e.tdu * (m[1] * r.x + m[2] * r.y + m[3] * r.z) +
+                   e.tdw * dot3(r, Lr) - tr * (e.tdw * s2 + 2.0 * e.tw) / 3.0;
+  w[0] += (k * r.x + e.tu * m[1] + 2.0 * e.tw * Lr.x) * r.x;
+  w[1] += (k * r.y + e.tu * m[2] + 2.0 * e.tw * Lr.y) * r.y;
+  w[2] += (k * r.z + e.tu * m[3] + 2.0 * e.tw * Lr.z) * r.z;
+}
+template <int W, int MB>
+__global__ void __launch_bounds__(W * 32, MB)
+pt_stress_kernel(PtArgs a, double F0, double F1, double F2, double *part, unsigned *count,
+                 int *err, double *out) {
+  __shared__ double sh[W][3];
+  __shared__ bool last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const V3<double> F = mk3<double>(F0, F1, F2);
+  double w[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int u = blockIdx.x * W + warp; u < a.n_real; u += gridDim.x * W) {
+    const double xu = a.xb[u].x;
+    if (xu < kMinOcc) continue;
+    const double4 qu = a.pos[u];
+    const int cu = a.code[u], nb0 = a.offs[u], end = a.offs[u + 1];
+    double m[10];
+#pragma unroll
+    for (int c = 0; c < 10; ++c) m[c] = 0.0;
+    PtEntry e[kPtHold];
+#pragma unroll
+    for (int k = 0; k < kPtHold; ++k) {
+      e[k] = pt_entry(a, F, nb0 + 32 * k + lane, end, qu, cu, xu);
+      pt_entry_sums(e[k], m);
+    }
+#pragma unroll 1
+    for (int p = nb0 + 32 * kPtHold + lane; p < end; p += 32)
+      pt_entry_sums(pt_entry(a, F, p, end, qu, cu, xu), m);
+#pragma unroll
+    for (int c = 0; c < 10; ++c) m[c] = wsum(m[c]);
+    double Fe, dF;
+    spline_vd(cu == 0 ? a.emb_mg : a.emb_h, m[0], Fe, dF);
+    m[0] = xu * dF;
+    const double tr = m[4] + m[5] + m[6];
+#pragma unroll
+    for (int k = 0; k < kPtHold; ++k) pt_entry_stress(e[k], m, tr, w);
+#pragma unroll 1
+    for (int p = nb0 + 32 * kPtHold + lane; p < end; p += 32)
+      pt_entry_stress(pt_entry(a, F, p, end, qu, cu, xu), m, tr, w);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) w[c] = wsum(w[c]);
+  if (lane == 0)
+    for (int c = 0; c < 3; ++c) sh[warp][c] = w[c];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int c = 0; c < 3; ++c) {
+      double v = sh[0][c];
+      for (int k = 1; k < W; ++k) v += sh[k][c];
+      part[3 * (size_t)blockIdx.x + c] = v;
+    }
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || warp != 0) return;
+  __threadfence();
+  for (int c = 0; c < 3; ++c) {
+    double v = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(part + 3 * (size_t)b + c);
+    v = wsum(v);
+    if (lane == 0) out[c] = v;
+  }
+  if (lane == 0) {
+    out[3] = (double)*err;
+    *err = 0;
+    *count = 0;
   }
 }
 
@@ -538,6 +683,24 @@ int pt_buffers(btam_system *s, PtLayout &L) {
 
 PtArgs pt_args(btam_system *s, const PtLayout &L);
 
+// Sum of W(a, a) over the sites at diag(F) q into w (host), with one wait.  The
+// partial sums lie in L.rec, the block count (zero on entry; every launch's
+// last block clears it again) and the results in L.part.
+constexpr int kStressWarps = 4, kStressBlocks = 3;  // per block; blocks per SM
+int pt_stress(btam_system *s, const PtLayout &L, const double F[3], double w[3]) {
+  int sms = 0;
+  BTAM_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  const int full = std::max(1, nblk(s->n_real, kStressWarps)), g = std::min(full, kStressBlocks * sms);
+  unsigned *count = reinterpret_cast<unsigned *>(L.part + 4);
+  pt_stress_kernel<kStressWarps, kStressBlocks><<<g, 32 * kStressWarps, 0, s->st>>>(
+      pt_args(s, L), F[0], F[1], F[2], L.rec, count, s->err, L.part);
+  BTAM_TRY(cudaGetLastError());
+  double h[4];
+  BTAM_TRY(copy_sync(h, L.part, sizeof(h), cudaMemcpyDeviceToHost, s->st));
+  for (int a = 0; a < 3; ++a) w[a] = h[a];
+  return status_from_bits((int)h[3]);
+}
+
 // Enqueues both passes and the totals on the system's stream.
 int pt_run(btam_system *s, const PtLayout &L) {
   const PtArgs a = pt_args(s, L);
@@ -777,6 +940,8 @@ int relax_stretch(btam_system *s, int form, double atol, double rtol, int max_it
   BTAM_TRY(dalloc(q0, s->st, s->n_real));
   BTAM_TRY(cudaMemcpyAsync(q0, s->pos, (size_t)s->n_real * sizeof(double4),
                            cudaMemcpyDeviceToDevice, s->st));
+  if (form == 0)  // pt_stress's block count
+    BTAM_TRY(cudaMemsetAsync(L.part + 4, 0, sizeof(double), s->st));
   const GhostBox box0 = s->box;
   int evals = 0;
   // Y_a(X) = (1/V0) sum_u dV_u/dF(a, a) at q = diag(F) q0, F_aa = X_a when
@@ -784,26 +949,29 @@ int relax_stretch(btam_system *s, int form, double atol, double rtol, int max_it
   auto residual = [&](const double X[3], double Y[3]) -> int {
     double Fx[3];
     for (int a = 0; a < 3; ++a) Fx[a] = X[a] > 0.0 ? X[a] : 1.0;
-    GhostBox bF;
-    int r = apply_stretch(s, q0, box0, Fx, bF);
-    double *dtot = L.tot;
-    if (r == BTAM_OK) {
-      if (form == 0) {
-        r = pt_run(s, L);
-      } else {
-        double *W = nullptr;
-        r = mf_stress_enqueue(s, form == 1 ? BTAM_FP64 : BTAM_FP32C, &W, &dtot);
-      }
+    // sum of W(a, a): the point forms straight from the unstretched positions,
+    // the mean-field stress at moved ones
+    double w[3];
+    int r;
+    if (form == 0) {
+      r = pt_stress(s, L, Fx, w);
+    } else {
+      GhostBox bF;
+      r = apply_stretch(s, q0, box0, Fx, bF);
+      double *W = nullptr, *dtot = nullptr;
+      if (r == BTAM_OK) r = mf_stress_enqueue(s, form == 1 ? BTAM_FP64 : BTAM_FP32C, &W, &dtot);
+      double tot[kPtTot];
+      if (r == BTAM_OK)
+        r = cuda_status(cudaMemcpyAsync(tot, dtot, sizeof(tot), cudaMemcpyDeviceToHost, s->st));
+      if (r == BTAM_OK) r = read_err(s);
+      if (r == BTAM_OK)
+        for (int a = 0; a < 3; ++a) w[a] = tot[2 + 4 * a];
     }
-    double tot[kPtTot];
-    if (r == BTAM_OK)
-      r = cuda_status(cudaMemcpyAsync(tot, dtot, sizeof(tot), cudaMemcpyDeviceToHost, s->st));
-    if (r == BTAM_OK) r = read_err(s);
     if (r != BTAM_OK) return r;
     ++evals;
     // W is taken at q0 = q; the reference's dV/dF(a, a) at the unstretched
     // q0 is W(a, a) / F_aa
-    for (int a = 0; a < 3; ++a) Y[a] = tot[2 + 4 * a] / (Fx[a] * vol);
+    for (int a = 0; a < 3; ++a) Y[a] = w[a] / (Fx[a] * vol);
     for (int a = 0; a < 3; ++a)
       if (!std::isfinite(Y[a])) return BTAM_ERR_NONFINITE;
     return BTAM_OK;
