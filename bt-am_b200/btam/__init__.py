@@ -399,8 +399,8 @@ class System:
 
     def evaluate(self, precision=FP64):
         n = self.n
-        out = dict(rho=np.zeros(n), V0=np.zeros(n), S0=np.zeros(n), Rq=np.zeros((n, 3)),
-                   Rs=np.zeros(n), Rx=np.zeros(n), totals=np.zeros(4))
+        out = dict(rho=np.empty(n), V0=np.empty(n), S0=np.empty(n), Rq=np.empty((n, 3)),
+                   Rs=np.empty(n), Rx=np.empty(n), totals=np.empty(4))
         _check(lib().btam_mf_eval(self.handle, precision, _d(out["rho"]), _d(out["V0"]),
                                   _d(out["S0"]), _d(out["Rq"]), _d(out["Rs"]), _d(out["Rx"]),
                                   _d(out["totals"])), "btam_mf_eval")
@@ -409,8 +409,8 @@ class System:
     def evaluate_state(self, precision=FP64, q=None, sigma=None, x=None):
         """New state and its evaluation in one call (btam_mf_eval_state)."""
         n = self.n
-        out = dict(rho=np.zeros(n), V0=np.zeros(n), S0=np.zeros(n), Rq=np.zeros((n, 3)),
-                   Rs=np.zeros(n), Rx=np.zeros(n), totals=np.zeros(4))
+        out = dict(rho=np.empty(n), V0=np.empty(n), S0=np.empty(n), Rq=np.empty((n, 3)),
+                   Rs=np.empty(n), Rx=np.empty(n), totals=np.empty(4))
         cv = lambda a: None if a is None else np.ascontiguousarray(a, np.float64)
         q, sigma, x = cv(q), cv(sigma), cv(x)
         _check(lib().btam_mf_eval_state(self.handle, precision, _d(q), _d(sigma), _d(x),
@@ -459,15 +459,15 @@ class System:
     def results(self, want=("V0", "Rq", "Rs", "Rx", "totals")):
         n = self.n
         shapes = dict(rho=(n,), V0=(n,), S0=(n,), Rq=(n, 3), Rs=(n,), Rx=(n,), totals=(4,))
-        out = {k: np.zeros(shapes[k]) for k in want}
+        out = {k: np.empty(shapes[k]) for k in want}
         args = [_d(out.get(k)) for k in ("rho", "V0", "S0", "Rq", "Rs", "Rx", "totals")]
         _check(lib().btam_results_copy(self.handle, *args), "btam_results_copy")
         return out
 
     def get_state(self):
-        q = np.zeros((self.n, 3))
-        sigma = np.zeros(self.n)
-        x = np.zeros(self.n)
+        q = np.empty((self.n, 3))
+        sigma = np.empty(self.n)
+        x = np.empty(self.n)
         _check(lib().btam_system_get_state(self.handle, _d(q), _d(sigma), _d(x)),
                "btam_system_get_state")
         return q, sigma, x
@@ -596,8 +596,8 @@ class System:
         Fq (n, 3) = sum_{i in {u} U N(u)} dV_i/dq_u, W (n, 3, 3) = dV_u/dF at
         q0 = q, totals (12): sum V, sum |Fq|^2, sum W (9), 0."""
         n = self.n
-        out = dict(rho=np.zeros(n), V=np.zeros(n), Fq=np.zeros((n, 3)), W=np.zeros((n, 3, 3)),
-                   totals=np.zeros(12))
+        out = dict(rho=np.empty(n), V=np.empty(n), Fq=np.empty((n, 3)), W=np.empty((n, 3, 3)),
+                   totals=np.empty(12))
         _check(lib().btam_pt_eval(self.handle, _d(out["rho"]), _d(out["V"]), _d(out["Fq"]),
                                   _d(out["W"]), _d(out["totals"])), "btam_pt_eval")
         return out

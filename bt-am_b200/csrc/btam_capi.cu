@@ -327,6 +327,237 @@ void release_state_slots(btam_system *s);
 
 }  // namespace
 
+namespace {
+
+// Doubles from one result array to the next in a system's result block.
+inline size_t result_stride(int n) { return ((size_t)n + 31) & ~(size_t)31; }
+
+// Planar q, sigma, x of the sites.
+__global__ void unpack_state_kernel(int n, const double4 *pos, const double2 *xb, double *q,
+                                    double *sigma, double *x) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double4 p = pos[i];
+  q[3 * (size_t)i] = p.x;
+  q[3 * (size_t)i + 1] = p.y;
+  q[3 * (size_t)i + 2] = p.z;
+  sigma[i] = p.w;
+  x[i] = xb[i].x;
+}
+
+// Pinned buffers of the calling thread for copies between a system's arrays and
+// the caller's pageable ones: 1 MB in four slots, made by the first such copy and
+// freed with the thread.  A cudaMemcpyAsync on pageable memory costs some 8 us
+// of calls and waits beside its bytes, so what fits one slot moves as one block;
+// larger results pass through the slots, the copy engine filling one while the
+// host empties another (27,000 sites' results: 216 -> 139 us).  Inputs larger
+// than a slot are as fast without it (106 us against 121).
+struct PinnedRing {
+  static constexpr int kSlots = 4;
+  static constexpr size_t kSlot = 32768;  // doubles
+  int device = -1;
+  double *buf = nullptr;
+  cudaEvent_t ev[kSlots] = {};
+  cudaStream_t st = nullptr;  // copies that pass the system's later kernels
+  cudaEvent_t part = nullptr;  // and what they wait for
+  unsigned next = 0;           // slots handed out so far
+  bool ready(int dev) {
+    if (buf && dev == device) return true;
+    release();
+    bool ok = cudaHostAlloc(&buf, kSlots * kSlot * sizeof(double), cudaHostAllocDefault) ==
+              cudaSuccess;
+    for (auto &e : ev)
+      ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaEventCreateWithFlags(&part, cudaEventDisableTiming) == cudaSuccess &&
+         cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+    if (ok) {
+      device = dev;
+      return true;
+    }
+    release();
+    cudaGetLastError();  // nothing is left to report: plain copies run
+    return false;
+  }
+  void release() {
+    for (auto &e : ev)
+      if (e) cudaEventDestroy(e);
+    if (part) cudaEventDestroy(part);
+    if (st) cudaStreamDestroy(st);
+    if (buf) cudaFreeHost(buf);
+    buf = nullptr;
+    part = nullptr;
+    st = nullptr;
+    for (auto &e : ev) e = nullptr;
+    device = -1;
+  }
+  // slot k may still be the source of another stream's copy: wait for its event
+  // before writing it (one that was never recorded counts as completed)
+  double *slot(unsigned k) { return buf + (k % kSlots) * kSlot; }
+  cudaEvent_t event(unsigned k) { return ev[k % kSlots]; }
+  ~PinnedRing() { release(); }
+};
+thread_local PinnedRing pinned_ring;
+
+// A served job copies once or twice in its life, on one of the server's
+// threads: making their slots took longer (a round of 48 jobs 26 -> 38 ms).
+inline bool ring_ready(const btam_system *s) {
+  return !s->served && pinned_ring.ready(s->device);
+}
+
+inline bool pinned(const void *p) {
+  cudaPointerAttributes a;
+  return cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+}
+
+}  // namespace
+cudaError_t copy_out(btam_system *s, const HostPiece *piece, int n_piece, cudaStream_t st) {
+  PinnedRing &r = pinned_ring;
+  const bool ring = ring_ready(s);
+  struct {
+    double *dst;
+    size_t count;
+  } out[PinnedRing::kSlots];
+  unsigned done = r.next;  // slots before this one are with the caller
+  auto take = [&]() -> cudaError_t {
+    const cudaError_t e = cudaEventSynchronize(r.event(done));
+    if (e != cudaSuccess) return e;
+    const auto &o = out[done % PinnedRing::kSlots];
+    std::memcpy(o.dst, r.slot(done++), o.count * sizeof(double));
+    return cudaSuccess;
+  };
+  bool direct = false;
+  for (int k = 0; k < n_piece; ++k) {
+    if (!piece[k].dst) continue;
+    if (!ring || pinned(piece[k].dst)) {
+      const cudaError_t e =
+          cudaMemcpyAsync(piece[k].dst, piece[k].dev, piece[k].count * sizeof(double),
+                          cudaMemcpyDeviceToHost, st);
+      if (e != cudaSuccess) return e;
+      direct = true;
+      continue;
+    }
+    // While the device still works, map the pages of an array that the caller
+    // has never touched: the byte written is the byte read.
+    volatile char *c = reinterpret_cast<volatile char *>(piece[k].dst);
+    for (size_t b = 0; b < piece[k].count * sizeof(double); b += 4096) c[b] = c[b];
+  }
+  for (int k = 0; ring && k < n_piece; ++k) {
+    if (!piece[k].dst || pinned(piece[k].dst)) continue;
+    for (size_t o = 0; o < piece[k].count; o += PinnedRing::kSlot) {
+      const size_t c = std::min(piece[k].count - o, PinnedRing::kSlot);
+      cudaError_t e = cudaSuccess;
+      if (r.next - done == PinnedRing::kSlots) e = take();
+      const unsigned id = r.next;
+      if (e == cudaSuccess) e = cudaEventSynchronize(r.event(id));
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(r.slot(id), piece[k].dev + o, c * sizeof(double),
+                            cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaEventRecord(r.event(id), st);
+      if (e != cudaSuccess) return e;
+      out[id % PinnedRing::kSlots] = {piece[k].dst + o, c};
+      ++r.next;
+    }
+  }
+  while (done != r.next) {
+    const cudaError_t e = take();
+    if (e != cudaSuccess) return e;
+  }
+  return direct ? cudaStreamSynchronize(st) : cudaSuccess;
+}
+
+namespace {
+
+// The same for pieces of one device block of `count` doubles that fits a slot.
+bool one_slot(btam_system *s, size_t count) {
+  return count <= PinnedRing::kSlot && ring_ready(s);
+}
+cudaError_t block_out(btam_system *s, const HostPiece *piece, int n_piece, const double *block,
+                      size_t count) {
+  PinnedRing &r = pinned_ring;
+  const unsigned id = r.next++;
+  cudaError_t e = cudaEventSynchronize(r.event(id));
+  if (e != cudaSuccess) return e;
+  e = copy_sync(r.slot(id), block, count * sizeof(double),
+                                  cudaMemcpyDeviceToHost, s->st);
+  if (e != cudaSuccess) return e;
+  for (int k = 0; k < n_piece; ++k)
+    if (piece[k].dst)
+      std::memcpy(piece[k].dst, r.slot(id) + (piece[k].dev - block),
+                  piece[k].count * sizeof(double));
+  return cudaSuccess;
+}
+
+// The wanted results, the error bits and the validation flags, with one wait;
+// the error bits are cleared on the device if there are any.  part: an event
+// after the kernels that made rho, V0 and S0, which then go out under the
+// others (null: none).
+cudaError_t results_out(btam_system *s, double *rho, double *V0, double *S0, double *Rq,
+                        double *Rs, double *Rx, double *totals, int (&bits)[2],
+                        cudaEvent_t part = nullptr) {
+  const size_t n = (size_t)s->n_real;
+  double word;
+  const HostPiece out[8] = {{rho, s->rho, n},       {V0, s->V0, n}, {S0, s->S0, n},
+                            {Rq, s->Rq, 3 * n},     {Rs, s->Rs, n}, {Rx, s->Rx, n},
+                            {totals, s->totals, 4}, {&word, s->totals + 4, 1}};
+  const size_t count = 8 * result_stride(s->n_real) + 5;
+  cudaError_t e = cudaSuccess;
+  if (one_slot(s, count)) {
+    e = block_out(s, out, 8, s->rho, count);
+  } else {
+    if (part) {
+      e = cudaStreamWaitEvent(pinned_ring.st, part, 0);
+      if (e == cudaSuccess) e = copy_out(s, out, 3, pinned_ring.st);
+    }
+    if (e == cudaSuccess) e = copy_out(s, out + (part ? 3 : 0), part ? 5 : 8, s->st);
+  }
+  if (e != cudaSuccess) return e;
+  std::memcpy(bits, &word, sizeof(bits));
+  return bits[0] ? cudaMemsetAsync(s->err, 0, sizeof(int), s->st) : cudaSuccess;
+}
+// That event, for a system whose results leave in pieces.
+cudaEvent_t part_event(btam_system *s) {
+  const bool pieces = !s->batcher && ring_ready(s) &&
+                      8 * result_stride(s->n_real) + 5 > PinnedRing::kSlot;
+  return pieces ? pinned_ring.part : nullptr;
+}
+
+// New q, sigma and x (null: unchanged) to the staging arrays.
+cudaError_t state_in(btam_system *s, const double *q, const double *sigma, const double *x) {
+  const size_t n = (size_t)s->n_real;
+  const struct {
+    const double *src;
+    size_t off, count;
+  } in[3] = {{q, 0, 3 * n}, {sigma, 3 * n, n}, {x, 4 * n, n}};
+  if (one_slot(s, 5 * n)) {
+    PinnedRing &r = pinned_ring;
+    const unsigned id = r.next;
+    cudaError_t e = cudaEventSynchronize(r.event(id));
+    if (e != cudaSuccess) return e;
+    double *b = r.slot(id);
+    size_t lo = 5 * n, hi = 0;
+    for (const auto &p : in)
+      if (p.src) {
+        std::memcpy(b + p.off, p.src, p.count * sizeof(double));
+        lo = std::min(lo, p.off);
+        hi = std::max(hi, p.off + p.count);
+      }
+    if (hi <= lo) return cudaSuccess;
+    ++r.next;
+    e = cudaMemcpyAsync(s->stage + lo, b + lo, (hi - lo) * sizeof(double),
+                        cudaMemcpyHostToDevice, s->st);
+    return e == cudaSuccess ? cudaEventRecord(r.event(id), s->st) : e;
+  }
+  for (const auto &p : in)
+    if (p.src) {
+      const cudaError_t e = cudaMemcpyAsync(s->stage + p.off, p.src, p.count * sizeof(double),
+                                            cudaMemcpyHostToDevice, s->st);
+      if (e != cudaSuccess) return e;
+    }
+  return cudaSuccess;
+}
+
+}  // namespace
+
 // One evaluation enqueued on the system's stream.  x_only: the occupancy
 // gradients alone with the undirected variants (EvalArgs::x_only); recs_ready:
 // the pair-rule kernel's four pass-1 sums are still those of the current
@@ -335,9 +566,9 @@ void release_state_slots(btam_system *s);
 // job's evaluation goes to the server's batcher in full.  totals: also the
 // system's totals (the solvers form their own sums and complete the totals
 // once, at the end).  kept: slot values of an x-only run (EvalArgs::kept), made
-// by its first evaluation.
+// by its first evaluation.  part: recorded once rho, V0 and S0 are made.
 static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_ready,
-                        bool totals = true, void *kept = nullptr) {
+                        bool totals = true, void *kept = nullptr, cudaEvent_t part = nullptr) {
   if (!s) return BTAM_ERR_ARG;
   if (!s->built) return BTAM_ERR_NOT_BUILT;
   if (precision != BTAM_FP64 && precision != BTAM_FP32C) return BTAM_ERR_ARG;
@@ -353,6 +584,7 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
     a.kept = static_cast<double *>(kept);
     a.n_slots = s->n_pairs;
     BTAM_TRY(launch_pass1(a, s->st, v1, v2));
+    if (part) BTAM_TRY(cudaEventRecord(part, s->st));
     BTAM_TRY(launch_pass2(a, s->st, v2));
   } else {
     if (!s->mom32) BTAM_TRY(dalloc(s->mom32, s->st, nm));
@@ -362,11 +594,11 @@ static int enqueue_eval(btam_system *s, int precision, bool x_only, bool recs_re
     a.kept = static_cast<float *>(kept);
     a.n_slots = s->n_pairs;
     BTAM_TRY(launch_pass1(a, s->st, v1, v2));
+    if (part) BTAM_TRY(cudaEventRecord(part, s->st));
     BTAM_TRY(launch_pass2(a, s->st, v2));
   }
   if (totals)
-    BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals,
-                           s->totals + 4, s->st));
+    BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->tot_part, s->st));
   return BTAM_OK;
 }
 
@@ -703,14 +935,24 @@ int btam_system_create(const btam_tables *t, int n, const double *q, const doubl
       else e = cudaMemsetAsync(s->gamma, 0, n * sizeof(double), s->st);
     }
     if (e == cudaSuccess) e = dalloc(s->stage, s->st, 5 * (size_t)n);
-    // err[0]: error bits of the kernels; err[1]: state-validation flags
-    if (e == cudaSuccess) e = dalloc(s->err, s->st, 2);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->err, 0, sizeof(int), s->st);
-    for (double **p : {&s->rho, &s->V0, &s->S0, &s->selfx, &s->Rs, &s->Rx})
-      if (e == cudaSuccess) e = dalloc(*p, s->st, n);
-    if (e == cudaSuccess) e = dalloc(s->Rq, s->st, 3 * (size_t)n);
-    // totals, then the partial sums of the two-stage totals reduction
-    if (e == cudaSuccess) e = dalloc(s->totals, s->st, 4 + 4 * kTotParts);
+    if (e == cudaSuccess) e = dalloc(s->selfx, s->st, n);
+    // the results in one block, so that a small system's go out in one copy:
+    // the arrays (each on a 256-byte boundary), the totals, the two error words
+    // (err[0]: error bits of the kernels; err[1]: state-validation flags), and
+    // behind them the partial sums of the two-stage totals reduction
+    const size_t stride = result_stride(n);
+    if (e == cudaSuccess) e = dalloc(s->rho, s->st, 8 * stride + 5 + 4 * kTotParts);
+    if (e == cudaSuccess) {
+      s->V0 = s->rho + stride;
+      s->S0 = s->V0 + stride;
+      s->Rs = s->S0 + stride;
+      s->Rx = s->Rs + stride;
+      s->Rq = s->Rx + stride;
+      s->totals = s->Rq + 3 * stride;
+      s->err = reinterpret_cast<int *>(s->totals + 4);
+      s->tot_part = s->totals + 5;
+      e = cudaMemsetAsync(s->err, 0, sizeof(int), s->st);
+    }
     if (e == cudaSuccess) e = dalloc(s->bbox, s->st, 6);
     if (e == cudaSuccess) e = dalloc(s->grid, s->st, 1);
     st = cuda_status(e);
@@ -732,9 +974,8 @@ void btam_system_destroy(btam_system *s) {
   dfree(s->s32, s->st); dfree(s->sb, s->st); dfree(s->s64, s->st);
   dfree(s->gamma, s->st); dfree(s->stage, s->st); dfree(s->offs, s->st); dfree(s->idx, s->st); dfree(s->cnt, s->st);
   dfree(s->tmp, s->st); dfree(s->bbox, s->st); dfree(s->grid, s->st); dfree(s->cell_of, s->st); dfree(s->cell_cnt, s->st);
-  dfree(s->cell_start, s->st); dfree(s->cursor, s->st); dfree(s->cell_sites, s->st); dfree(s->rho, s->st); dfree(s->V0, s->st);
-  dfree(s->S0, s->st); dfree(s->selfx, s->st); dfree(s->Rq, s->st); dfree(s->Rs, s->st); dfree(s->Rx, s->st); dfree(s->totals, s->st);
-  dfree(s->mom64, s->st); dfree(s->mom32, s->st); dfree(s->err, s->st);
+  dfree(s->cell_start, s->st); dfree(s->cursor, s->st); dfree(s->cell_sites, s->st); dfree(s->rho, s->st); dfree(s->selfx, s->st);
+  dfree(s->mom64, s->st); dfree(s->mom32, s->st);
   dfree(s->doffs, s->st); dfree(s->didx, s->st); dfree(s->X, s->st); dfree(s->X0, s->st); dfree(s->dtot, s->st); dfree(s->mu, s->st);
   dfree(s->dctl, s->st);
   dfree(s->dact, s->st); dfree(s->dout, s->st); dfree(s->din, s->st); dfree(s->rv, s->st);
@@ -753,9 +994,7 @@ int btam_system_set_state(btam_system *s, const double *q, const double *sigma,
   // validate_state); the device keeps the old state if it is rejected
   const int n = s->n_real;
   double *dq = s->stage, *ds = s->stage + 3 * (size_t)n, *dx = s->stage + 4 * (size_t)n;
-  if (q) BTAM_TRY(cudaMemcpyAsync(dq, q, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s->st));
-  if (sigma) BTAM_TRY(cudaMemcpyAsync(ds, sigma, n * sizeof(double), cudaMemcpyHostToDevice, s->st));
-  if (x) BTAM_TRY(cudaMemcpyAsync(dx, x, n * sizeof(double), cudaMemcpyHostToDevice, s->st));
+  BTAM_TRY(state_in(s, q, sigma, x));
   if (!q && !sigma && !x) return BTAM_OK;
   BTAM_TRY(cudaMemsetAsync(s->err + 1, 0, sizeof(int), s->st));
   validate_stage_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(
@@ -1041,25 +1280,21 @@ int btam_system_sync(btam_system *s) {
 int btam_results_copy(btam_system *s, double *rho, double *V0, double *S0, double *Rq,
                       double *Rs, double *Rx, double *totals) {
   if (!s) return BTAM_ERR_ARG;
-  const size_t n = (size_t)s->n_real * sizeof(double);
-  struct {
-    double *dst;
-    const double *src;
-    size_t bytes;
-  } cp[7] = {{rho, s->rho, n}, {V0, s->V0, n}, {S0, s->S0, n}, {Rq, s->Rq, 3 * n},
-             {Rs, s->Rs, n},   {Rx, s->Rx, n}, {totals, s->totals, 4 * sizeof(double)}};
-  for (auto &c : cp)
-    if (c.dst) BTAM_TRY(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, s->st));
-  return read_err(s);
+  int bits[2] = {0, 0};
+  BTAM_TRY(results_out(s, rho, V0, S0, Rq, Rs, Rx, totals, bits));
+  return status_from_bits(bits[0]);
 }
 
 int btam_mf_eval(btam_system *s, int precision, double *rho, double *V0, double *S0,
                  double *Rq, double *Rs, double *Rx, double *totals) {
   if (!s) return BTAM_ERR_ARG;
   BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
-  int st = btam_mf_eval_async(s, precision);
+  const cudaEvent_t part = part_event(s);
+  int st = enqueue_eval(s, precision, false, false, true, nullptr, part);
   if (st != BTAM_OK) return st;
-  return btam_results_copy(s, rho, V0, S0, Rq, Rs, Rx, totals);
+  int bits[2] = {0, 0};
+  BTAM_TRY(results_out(s, rho, V0, S0, Rq, Rs, Rx, totals, bits, part));
+  return status_from_bits(bits[0]);
 }
 
 int btam_mf_eval_state(btam_system *s, int precision, const double *q, const double *sigma,
@@ -1073,9 +1308,7 @@ int btam_mf_eval_state(btam_system *s, int precision, const double *q, const dou
   // the host waits once
   const int n = s->n_real;
   double *dq = s->stage, *ds = s->stage + 3 * (size_t)n, *dx = s->stage + 4 * (size_t)n;
-  if (q) BTAM_TRY(cudaMemcpyAsync(dq, q, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s->st));
-  if (sigma) BTAM_TRY(cudaMemcpyAsync(ds, sigma, n * sizeof(double), cudaMemcpyHostToDevice, s->st));
-  if (x) BTAM_TRY(cudaMemcpyAsync(dx, x, n * sizeof(double), cudaMemcpyHostToDevice, s->st));
+  BTAM_TRY(state_in(s, q, sigma, x));
   BTAM_TRY(cudaMemsetAsync(s->err, 0, 2 * sizeof(int), s->st));
   if (q || sigma || x) {
     validate_stage_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(
@@ -1088,23 +1321,12 @@ int btam_mf_eval_state(btam_system *s, int precision, const double *q, const dou
       BTAM_TRY(launch_ghost_refresh(n, s->n_ghost, s->pos, s->xb, s->code, s->owner, s->image,
                                     s->box, s->st));
   }
-  int st = btam_mf_eval_async(s, precision);
+  const cudaEvent_t part = part_event(s);
+  int st = enqueue_eval(s, precision, false, false, true, nullptr, part);
   if (st != BTAM_OK) return st;
-  // the result copies, then the validation flags and error bits behind
-  // them, and one wait for all of it
-  const size_t nb = (size_t)n * sizeof(double);
-  const struct {
-    double *dst;
-    const double *src;
-    size_t bytes;
-  } cp[7] = {{rho, s->rho, nb}, {V0, s->V0, nb}, {S0, s->S0, nb}, {Rq, s->Rq, 3 * nb},
-             {Rs, s->Rs, nb},   {Rx, s->Rx, nb}, {totals, s->totals, 4 * sizeof(double)}};
-  for (const auto &c : cp)
-    if (c.dst) BTAM_TRY(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, s->st));
+  // the results, with the validation flags and the error bits
   int bits[2] = {0, 0};
-  BTAM_TRY(cudaMemcpyAsync(bits, s->err, 2 * sizeof(int), cudaMemcpyDeviceToHost, s->st));
-  BTAM_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
-  BTAM_TRY(cudaStreamSynchronize(s->st));
+  BTAM_TRY(results_out(s, rho, V0, S0, Rq, Rs, Rx, totals, bits, part));
   const int flags = bits[1];
   st = status_from_bits(bits[0]);
   if (flags & 1) return BTAM_ERR_NONFINITE;
@@ -1313,7 +1535,7 @@ int btam_mf_eval_profile(btam_system *s, int precision, double ms[5]) {
   }
   if (e == cudaSuccess) e = cudaEventRecord(ev[4], s->st);
   if (e == cudaSuccess)
-    e = launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->totals + 4,
+    e = launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->tot_part,
                       s->st);
   if (e == cudaSuccess) e = cudaEventRecord(ev[5], s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
@@ -1563,7 +1785,7 @@ int relax_eval(btam_system *s, int prec, RelaxVecs &v, double &f, double &r2,
 // The totals of the last evaluation (a served one brought its own).
 int relax_totals(btam_system *s) {
   if (s->batcher) return BTAM_OK;
-  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->totals + 4,
+  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->tot_part,
                          s->st));
   return BTAM_OK;
 }
@@ -2289,16 +2511,19 @@ int btam_dmd_occupancy(btam_system *s, double *x, long long *quanta, double *mu)
   if (!s) return BTAM_ERR_ARG;
   if (!s->dmd_ready) return BTAM_ERR_NOT_BUILT;
   const int n = s->n_real;
-  if (quanta)
-    BTAM_TRY(cudaMemcpyAsync(quanta, s->X, n * sizeof(long long), cudaMemcpyDeviceToHost, s->st));
-  if (mu) BTAM_TRY(cudaMemcpyAsync(mu, s->mu, n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
+  double *dx = s->stage + 4 * (size_t)n, word;
   if (x) {
-    std::vector<double2> h(n);
-    BTAM_TRY(cudaMemcpyAsync(h.data(), s->xb, n * sizeof(double2), cudaMemcpyDeviceToHost, s->st));
-    BTAM_TRY(cudaStreamSynchronize(s->st));
-    for (int i = 0; i < n; ++i) x[i] = h[i].x;
+    unpack_state_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(
+        n, s->pos, s->xb, s->stage, s->stage + 3 * (size_t)n, dx);
+    BTAM_TRY(cudaGetLastError());
   }
-  return read_err(s);
+  const HostPiece out[4] = {
+      {reinterpret_cast<double *>(quanta), reinterpret_cast<double *>(s->X), (size_t)n},
+      {mu, s->mu, (size_t)n},
+      {x, dx, (size_t)n},
+      {&word, s->totals + 4, 1}};
+  BTAM_TRY(copy_out(s, out, 4, s->st));
+  return take_err(s, word);
 }
 
 int btam_dmd_graph_copy(const btam_system *s, int *offs, int *idx, long long idx_cap) {
@@ -2314,22 +2539,18 @@ int btam_dmd_graph_copy(const btam_system *s, int *offs, int *idx, long long idx
 
 int btam_system_get_state(btam_system *s, double *q, double *sigma, double *x) {
   if (!s) return BTAM_ERR_ARG;
-  const int n = s->n_real;
-  std::vector<double4> hp(n);
-  std::vector<double2> hx(n);
-  BTAM_TRY(cudaMemcpyAsync(hp.data(), s->pos, n * sizeof(double4), cudaMemcpyDeviceToHost, s->st));
-  BTAM_TRY(cudaMemcpyAsync(hx.data(), s->xb, n * sizeof(double2), cudaMemcpyDeviceToHost, s->st));
-  BTAM_TRY(cudaStreamSynchronize(s->st));
-  for (int i = 0; i < n; ++i) {
-    if (q) {
-      q[3 * i] = hp[i].x;
-      q[3 * i + 1] = hp[i].y;
-      q[3 * i + 2] = hp[i].z;
-    }
-    if (sigma) sigma[i] = hp[i].w;
-    if (x) x[i] = hx[i].x;
+  if (!q && !sigma && !x) {
+    BTAM_TRY(cudaStreamSynchronize(s->st));
+    return BTAM_OK;
   }
-  return BTAM_OK;
+  const int n = s->n_real;
+  double *dq = s->stage, *ds = s->stage + 3 * (size_t)n, *dx = s->stage + 4 * (size_t)n;
+  unpack_state_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(n, s->pos, s->xb, dq, ds, dx);
+  BTAM_TRY(cudaGetLastError());
+  const HostPiece out[3] = {{q, dq, 3 * (size_t)n}, {sigma, ds, (size_t)n}, {x, dx, (size_t)n}};
+  return cuda_status(one_slot(s, 5 * (size_t)n)
+                         ? block_out(s, out, 3, s->stage, 5 * (size_t)n)
+                         : copy_out(s, out, 3, s->st));
 }
 
 }  // extern "C"

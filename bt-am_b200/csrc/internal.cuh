@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <utility>
 #include <vector>
 
@@ -67,7 +68,7 @@ struct btam_system {
       *cell_sites = nullptr;
   // results
   double *rho = nullptr, *V0 = nullptr, *S0 = nullptr, *selfx = nullptr, *Rq = nullptr,
-         *Rs = nullptr, *Rx = nullptr, *totals = nullptr;
+         *Rs = nullptr, *Rx = nullptr, *totals = nullptr, *tot_part = nullptr;
   double *mom64 = nullptr;
   float *mom32 = nullptr;
   int *err = nullptr;
@@ -95,6 +96,7 @@ struct btam_system {
   int own_off_cap = 0, n_own = 0;
   int n_unpaired = 0;      // entries without a reverse (rev < 0)
   bool same_beta = false;  // every site has the same beta
+  bool served = false;  // a server's job
   // most bytes a master-equation call may take for kept slot values
   size_t kept_limit = (size_t)-1;
   char *pbuf = nullptr;
@@ -158,6 +160,16 @@ cudaError_t launch_pt_totals(int n, const double *V, const double *Fq, const dou
 // Enqueues the FP64 directed pass 1: the mean-field rho-bar, V0 and S0 of
 // the current state into the system's buffers (btam_capi.cu).
 int mf_rho64_enqueue(btam_system *s);
+
+// A piece of a device array and where it goes on the host (null: unwanted).
+struct HostPiece {
+  double *dst;
+  const double *dev;
+  size_t count;
+};
+// The pieces to the host, the last of them there on return.  st: the stream
+// that makes them (btam_capi.cu).
+cudaError_t copy_out(btam_system *s, const HostPiece *piece, int n_piece, cudaStream_t st);
 
 // Enqueues the mean-field Hessian blocks of the current state into Hd (9
 // per real site); with Hslot (9 per entry of the real sites' lists), Hd
@@ -264,10 +276,19 @@ inline cudaError_t copy_sync(void *dst, const void *src, size_t bytes, cudaMemcp
 // (as a status) and clears them.
 inline int read_err(btam_system *s) {
   int bits = 0;
-  cudaError_t e = cudaMemcpyAsync(&bits, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s->err, 0, sizeof(int), s->st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+  cudaError_t e = copy_sync(&bits, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->st);
+  if (e == cudaSuccess && bits) e = cudaMemsetAsync(s->err, 0, sizeof(int), s->st);
   if (e != cudaSuccess) return cuda_status(e);
+  return status_from_bits(bits);
+}
+// The same for the error words (s->totals + 4) already read with other results.
+inline int take_err(btam_system *s, double word) {
+  int bits;
+  std::memcpy(&bits, &word, sizeof(bits));
+  if (bits) {
+    const cudaError_t e = cudaMemsetAsync(s->err, 0, sizeof(int), s->st);
+    if (e != cudaSuccess) return cuda_status(e);
+  }
   return status_from_bits(bits);
 }
 

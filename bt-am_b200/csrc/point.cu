@@ -825,14 +825,11 @@ int btam_pt_eval(btam_system *s, double *rho, double *V, double *Fq, double *W,
   if (st != BTAM_OK) return st;
   if ((st = pt_run(s, L)) != BTAM_OK) return st;
   const size_t n = (size_t)s->n_real;
-  if (rho) BTAM_TRY(cudaMemcpyAsync(rho, L.rho, n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  if (V) BTAM_TRY(cudaMemcpyAsync(V, L.V, n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  if (Fq) BTAM_TRY(cudaMemcpyAsync(Fq, L.Fq, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  if (W) BTAM_TRY(cudaMemcpyAsync(W, L.W, 9 * n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  if (totals)
-    BTAM_TRY(cudaMemcpyAsync(totals, L.tot, kPtTot * sizeof(double), cudaMemcpyDeviceToHost,
-                             s->st));
-  return read_err(s);
+  double word;
+  const HostPiece out[6] = {{rho, L.rho, n},   {V, L.V, n},           {Fq, L.Fq, 3 * n},
+                            {W, L.W, 9 * n},   {totals, L.tot, kPtTot}, {&word, s->totals + 4, 1}};
+  BTAM_TRY(copy_out(s, out, 6, s->st));
+  return take_err(s, word);
 }
 
 int btam_pt_hessian(btam_system *s, double *H) {

@@ -307,6 +307,7 @@ void run_job(btam_server *srv, Job *job) {
                               job->species.data(), job->beta.empty() ? nullptr : job->beta.data(),
                               job->gamma.empty() ? nullptr : job->gamma.data(), job->origin,
                               job->cell, job->periodic, &s);
+  if (st == BTAM_OK) s->served = true;
   if (st == BTAM_OK) st = btam_neighbors_build(s, 0);
   // small jobs hand their evaluations to the batcher (the undirected
   // kernels on persistent grids, in the batch's buffers, which
