@@ -1160,9 +1160,7 @@ static int build_list(btam_system *s, int n_all, int n_query, double rc, int max
     BTAM_TRY(dalloc(idx, s->st, total));
     idx_cap = total;
   }
-  BTAM_TRY(launch_compact(n_query, s->tmp, offs, idx, s->st));
-  BTAM_TRY(cudaStreamSynchronize(s->st));
-  return BTAM_OK;
+  return cuda_status(launch_compact(n_query, s->tmp, offs, idx, s->st));
 }
 
 extern "C" {

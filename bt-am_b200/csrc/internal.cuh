@@ -64,8 +64,8 @@ struct btam_system {
   int cell_cap = 0, site_cap = 0;
   unsigned long long *bbox = nullptr;
   CellGrid *grid = nullptr;
-  int *cell_of = nullptr, *cell_cnt = nullptr, *cell_start = nullptr, *cursor = nullptr,
-      *cell_sites = nullptr;
+  int *cell_of = nullptr, *cell_cnt = nullptr, *cell_start = nullptr, *cursor = nullptr;
+  double4 *cell_sites = nullptr;
   // results
   double *rho = nullptr, *V0 = nullptr, *S0 = nullptr, *selfx = nullptr, *Rq = nullptr,
          *Rs = nullptr, *Rx = nullptr, *totals = nullptr, *tot_part = nullptr;

@@ -430,14 +430,14 @@ long long btam_estimate_bytes(int n, const double cell[9], const int periodic[3]
   }
   const double n_all = n * grow;
   // per all-sites row: position, occupancy/beta, species, owner, cell index,
-  // cell slot, image code; per real site: state, staging, results, both
+  // row in cell order, image code; per real site: state, staging, results, both
   // moment records, neighbour counts, the neighbour candidate buffer, the
   // neighbour list at the cap, master-equation state and graph, relaxation
   // vectors, and the undirected kernels' buffers at the cap (per slot:
   // reverse slot, owned-pair link and an FP64 slot record; per owned pair,
   // at most one per two slots: the pair and site indices and an FP64
   // pair-rule record); plus a fixed allowance for cells and library scratch
-  const double per_all = 32 + 16 + 4 + 4 + 4 + 4 + 4;
+  const double per_all = 32 + 16 + 4 + 4 + 4 + 32 + 4;
   const double per_slot = kSlotBytes;
   const double per_real = 8 + 40 + 48 + 24 + btam::kMomStride * 8 + btam::kMomStride * 4 + 8 + 256 * 4 +
                           BTAM_MAXNEIGH * 4 + 16 + 16 + 4 + BTAM_MAX_CHEMICAL_NEIGHS * 4 +

@@ -82,15 +82,16 @@ struct NbrArgs {
   const double4 *pos;
   unsigned long long *bbox;  // 6
   CellGrid *grid;
-  int *cell_of, *cell_cnt, *cell_start, *cursor, *cell_sites;
+  int *cell_of, *cell_cnt, *cell_start, *cursor;
+  double4 *cell_sites;  // n_all, in cell order
   int *cnt;   // n_query + 1
   int *tmp;   // n_query * kNbrBuf
   int *offs;  // n_query + 1
   int *err;
   DeviceScratch *scratch;
+  const int *code = nullptr;
   // optional restriction to one species code (-1: all sites), e.g. the H-H
   // diffusive graph; allow_empty = 1 accepts sites with no neighbour
-  const int *code = nullptr;
   int filter_code = -1;
   int allow_empty = 0;
 };
