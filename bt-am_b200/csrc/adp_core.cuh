@@ -510,6 +510,23 @@ BTAM_HD void pr_at(const RadialView<R> &T, int pk, int ci, int cj, int m, R p, R
   ri = ih ? r1 : r0;
   dri = ih ? dr1 : dr0;
 }
+// phi' and the density of species cj at its argument with its slope: the two
+// pieces of the record that hold them, whichever the kind.
+BTAM_HD void pr_slopes(const RadialView<double> &T, int pk, int cj, int m, double p, double &dph,
+                       double &rj, double &drj) {
+  double a[4], b[4], v;
+#if defined(__CUDA_ARCH__)
+  const int r = T.n * pk + m, o = pk == 2 && cj == 1 ? 2 : 1;
+  const double *q = T.prx + (pk == 2 ? (size_t)16 * (T.n + m) : (size_t)8 * r);
+  ld4(q + 4 * (pk == 2 ? rec128_piece(m, 0) : rec64_piece(r, 0)), a);
+  ld4(q + 4 * (pk == 2 ? rec128_piece(m, o) : rec64_piece(r, o)), b);
+#else
+  ld4(pr_rec(T, pk, m), a);
+  ld4(pr_rec(T, pk, m) + (pk == 2 && cj == 1 ? 8 : 4), b);
+#endif
+  cub_vd(a, p, v, dph);
+  cub_vd(b, p, rj, drj);
+}
 
 // A dual prepared for the six geometries r0 + a e_k that move along one
 // axis: Lambda r, r^T Lambda r and Da.r at r0, so each displaced geometry

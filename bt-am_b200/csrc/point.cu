@@ -236,16 +236,16 @@ __global__ void __launch_bounds__(128) pt_grad_kernel(PtArgs a, double *slot3) {
 // else of the point forms.  W_u depends on u's own list and moments alone, so
 // one warp per site does both: each lane looks its entries' splines up once,
 // the warp sums rho, mu and Lambda, and the lanes add g(u->j)_a r_a of the
-// entries, which they still hold (kPtHold a lane; the entries of a longer list
-// are looked up a second time).  A lane carries its three sums over all its
-// sites; the last block adds the blocks' partials in their order and hands the
-// error bits over with the sums.  Against the two passes over the lists, the
-// per-site outputs and their totals (81 + 156 + 11 us for 27,000 sites, and 4
-// for moving the sites and images first) it takes 125 us.  The lookups' L1
-// traffic and latency bound it: 4 entries a lane hold the usual list (up to 128)
-// in 164 registers, three blocks of 4 warps an SM.  5 entries at two blocks took
-// 156 us; 2 entries at four blocks (lists over 64 looked up twice) 127.
-constexpr int kPtHold = 4;
+// entries, which they still hold (2, 4 or kPtHold a lane, by the list's length;
+// the entries beyond are looked up a second time).  A lane carries its three
+// sums over all its sites; the last block adds the blocks' partials in their
+// order and hands the error bits over with the sums.  Against the two passes
+// over the lists, the per-site outputs and their totals (81 + 156 + 11 us for
+// 27,000 sites of 132 entries, and 4 for moving the sites and images first) it
+// takes 99 us.  The chains of loads (index, site, table pieces) bound it: one
+// entry after the other took 125 us; 4 held, and so a fifth of each list
+// looked up twice, 106; 5 held in 255 registers at two blocks an SM, 116.
+constexpr int kPtHold = 5;
 struct PtEntry {
   V3<double> r;
   double A, B;    // x_j rho'/s, t phi' / (2 s)
@@ -253,31 +253,41 @@ struct PtEntry {
   double tw, tdw; // t w, t w'/s
   double rho;     // x_j rho
 };
-__device__ __forceinline__ PtEntry pt_entry(const PtArgs &a, const V3<double> &F, int p, int end,
-                                            const double4 &qi, int ci, double xi) {
-  PtEntry e;
-  e.r = mk3<double>(0.0, 0.0, 0.0);
-  e.A = e.B = e.tu = e.tdu = e.tw = e.tdw = e.rho = 0.0;
-  if (p >= end) return e;
-  const int j = a.idx[p];
-  const double xj = a.xb[j].x;
-  if (xj < kMinOcc) return e;
-  const double4 qj = a.pos[j];
-  const int cj = a.code[j], pk = pair_kind(ci, cj);
-  e.r = mk3<double>(F.x * (qj.x - qi.x), F.y * (qj.y - qi.y), F.z * (qj.z - qi.z));
-  Geo<double> g;
-  double pp, ph, dph, rj, drj, ri, dri;
-  const int m = geo_uw<double, true>(g, e.r, a.T, pk, pp);
-  pr_at<double, true, false>(a.T, pk, ci, cj, m, pp, ph, dph, rj, drj, ri, dri);
-  const double t = xi * xj;
-  e.A = xj * drj * g.inv_s;
-  e.B = 0.5 * (t * dph) * g.inv_s;
-  e.tu = t * g.u;
-  e.tdu = t * g.du * g.inv_s;
-  e.tw = t * g.w;
-  e.tdw = t * g.dw * g.inv_s;
-  e.rho = xj * rj;
-  return e;
+// K entries a lane: 32 k + lane from p0 on; those past the list (end > p0), and
+// empty neighbours, weigh nothing.  No branch stands between the K chains of
+// loads (index, site, table pieces), so they run side by side.
+template <int K>
+__device__ __forceinline__ void pt_entries(const PtArgs &a, const V3<double> &F, int p0, int end,
+                                           const double4 &qi, int ci, double xi,
+                                           PtEntry (&e)[K]) {
+  int j[K], cj[K];
+  double xj[K];
+  double4 qj[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) j[k] = a.idx[min(p0 + 32 * k, end - 1)];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    xj[k] = a.xb[j[k]].x;
+    qj[k] = a.pos[j[k]];
+    cj[k] = a.code[j[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double x = p0 + 32 * k < end && !(xj[k] < kMinOcc) ? xj[k] : 0.0, t = xi * x;
+    const int pk = pair_kind(ci, cj[k]);
+    e[k].r = mk3<double>(F.x * (qj[k].x - qi.x), F.y * (qj[k].y - qi.y), F.z * (qj[k].z - qi.z));
+    Geo<double> g;
+    double pp, dph, rj, drj;
+    const int m = geo_uw<double, true>(g, e[k].r, a.T, pk, pp);
+    pr_slopes(a.T, pk, cj[k], m, pp, dph, rj, drj);
+    e[k].A = x * drj * g.inv_s;
+    e[k].B = 0.5 * (t * dph) * g.inv_s;
+    e[k].tu = t * g.u;
+    e[k].tdu = t * g.du * g.inv_s;
+    e[k].tw = t * g.w;
+    e[k].tdw = t * g.dw * g.inv_s;
+    e[k].rho = x * rj;
+  }
 }
 __device__ __forceinline__ void pt_entry_sums(const PtEntry &e, double (&m)[10]) {
   m[0] += e.rho;
@@ -306,6 +316,39 @@ __device__ __forceinline__ void pt_entry_stress(const PtEntry &e, const double (
   w[1] += (k * r.y + e.tu * m[2] + 2.0 * e.tw * Lr.y) * r.y;
   w[2] += (k * r.z + e.tu * m[3] + 2.0 * e.tw * Lr.z) * r.z;
 }
+// Site u's share of the three sums, K entries of its list a lane (a list longer
+// than 32 K is looked up twice beyond them).
+template <int K>
+__device__ __forceinline__ void pt_site_stress(const PtArgs &a, const V3<double> &F, int u,
+                                               double xu, int nb0, int end, double (&w)[3]) {
+  const int lane = threadIdx.x & 31, cu = a.code[u];
+  const double4 qu = a.pos[u];
+  double m[10];
+#pragma unroll
+  for (int c = 0; c < 10; ++c) m[c] = 0.0;
+  PtEntry e[K], f[1];
+  pt_entries<K>(a, F, nb0 + lane, end, qu, cu, xu, e);
+#pragma unroll
+  for (int k = 0; k < K; ++k) pt_entry_sums(e[k], m);
+#pragma unroll 1
+  for (int p = nb0 + 32 * K; p < end; p += 32) {
+    pt_entries<1>(a, F, p + lane, end, qu, cu, xu, f);
+    pt_entry_sums(f[0], m);
+  }
+#pragma unroll
+  for (int c = 0; c < 10; ++c) m[c] = wsum(m[c]);
+  double Fe, dF;
+  spline_vd(cu == 0 ? a.emb_mg : a.emb_h, m[0], Fe, dF);
+  m[0] = xu * dF;
+  const double tr = m[4] + m[5] + m[6];
+#pragma unroll
+  for (int k = 0; k < K; ++k) pt_entry_stress(e[k], m, tr, w);
+#pragma unroll 1
+  for (int p = nb0 + 32 * K; p < end; p += 32) {
+    pt_entries<1>(a, F, p + lane, end, qu, cu, xu, f);
+    pt_entry_stress(f[0], m, tr, w);
+  }
+}
 template <int W, int MB>
 __global__ void __launch_bounds__(W * 32, MB)
 pt_stress_kernel(PtArgs a, double F0, double F1, double F2, double *part, unsigned *count,
@@ -319,31 +362,10 @@ pt_stress_kernel(PtArgs a, double F0, double F1, double F2, double *part, unsign
   for (int u = blockIdx.x * W + warp; u < a.n_real; u += gridDim.x * W) {
     const double xu = a.xb[u].x;
     if (xu < kMinOcc) continue;
-    const double4 qu = a.pos[u];
-    const int cu = a.code[u], nb0 = a.offs[u], end = a.offs[u + 1];
-    double m[10];
-#pragma unroll
-    for (int c = 0; c < 10; ++c) m[c] = 0.0;
-    PtEntry e[kPtHold];
-#pragma unroll
-    for (int k = 0; k < kPtHold; ++k) {
-      e[k] = pt_entry(a, F, nb0 + 32 * k + lane, end, qu, cu, xu);
-      pt_entry_sums(e[k], m);
-    }
-#pragma unroll 1
-    for (int p = nb0 + 32 * kPtHold + lane; p < end; p += 32)
-      pt_entry_sums(pt_entry(a, F, p, end, qu, cu, xu), m);
-#pragma unroll
-    for (int c = 0; c < 10; ++c) m[c] = wsum(m[c]);
-    double Fe, dF;
-    spline_vd(cu == 0 ? a.emb_mg : a.emb_h, m[0], Fe, dF);
-    m[0] = xu * dF;
-    const double tr = m[4] + m[5] + m[6];
-#pragma unroll
-    for (int k = 0; k < kPtHold; ++k) pt_entry_stress(e[k], m, tr, w);
-#pragma unroll 1
-    for (int p = nb0 + 32 * kPtHold + lane; p < end; p += 32)
-      pt_entry_stress(pt_entry(a, F, p, end, qu, cu, xu), m, tr, w);
+    const int nb0 = a.offs[u], end = a.offs[u + 1];
+    if (end - nb0 > 128) pt_site_stress<kPtHold>(a, F, u, xu, nb0, end, w);
+    else if (end - nb0 > 64) pt_site_stress<4>(a, F, u, xu, nb0, end, w);
+    else if (end > nb0) pt_site_stress<2>(a, F, u, xu, nb0, end, w);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) w[c] = wsum(w[c]);

@@ -1,8 +1,8 @@
 """The stretch relaxation's residual (pt_stress_kernel) against the point forms'
 per-site stress of the stretched system.
 
-Forms: periodic and open; empty sites; lists from a few entries to more than
-one warp holds (128); fewer sites than one block and more than one round of the
+Forms: periodic and open; empty sites; lists of a few entries, up to 64, up to 128
+and beyond what a warp holds (160); fewer sites than one block and more than one round of the
 grid.  No iteration is taken, so the reported norm is that of the residual at
 F0, and the system is left stretched by F0, where pt_eval gives the per-site
 stress.  Both sum the same FP64 terms in another order, and form r as
@@ -29,6 +29,8 @@ SYSTEMS = {
                                               jitter=0.02, seed=31)),
     "full_cell": lambda: lattice.supercell(14, 10, 8, h_fraction=1.0, x_range=(0.2, 0.9),
                                            jitter=0.02, seed=32),
+    "dense_cell": lambda: lattice.supercell(9, 8, 7, h_fraction=1.0, x_range=(0.2, 0.9), a=2.75,
+                                            jitter=0.01, seed=35),
     "sphere": lambda: lattice.cluster("sphere", 5.0, h_fraction=0.5, seed=33),
     "few": lambda: lattice.cluster("sphere", 3.5, h_fraction=0.0, seed=34),
 }
