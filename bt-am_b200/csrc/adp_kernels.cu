@@ -443,23 +443,28 @@ template <int NSITES> __host__ __device__ constexpr int p1_cache_cap() {
   return room > 136 ? 136 : (room < 0 ? 0 : room);
 }
 
-template <class R, int W, int MB, int G, bool UND>
+template <class R, int W, int MB, int G, bool UND, bool SPLIT = false>
 __global__ void __launch_bounds__(W * 32, MB)
 pass1_kernel(const EvalArgs<R> a) {
   constexpr int SPW = 32 / G;  // sites per warp
-  __shared__ SiteSums ss[W * SPW];
-  constexpr int kCap = sizeof(R) == 8 ? p1_cache_cap<W * SPW>() : 0;
-  __shared__ double4 rx_s[kCap > 0 ? W * SPW * kCap : 1];  // (r0, X) per cached slot
-  __shared__ signed char pk_s[kCap > 0 ? W * SPW * kCap : 1];  // pair kind, -1: inactive
+  constexpr int NS = SPLIT ? 1 : W * SPW;  // sites a block holds at once
+  static_assert(!SPLIT || (SPW == 1 && W == (sizeof(R) == 8 ? 4 : 2)), "a warp per part");
+  __shared__ SiteSums ss[NS];
+  __shared__ double sself_s[SPLIT ? 3 : 1];
+  constexpr int kCap = sizeof(R) == 8 && !SPLIT ? p1_cache_cap<NS>() : 0;
+  __shared__ double4 rx_s[kCap > 0 ? NS * kCap : 1];  // (r0, X) per cached slot
+  __shared__ signed char pk_s[kCap > 0 ? NS * kCap : 1];  // pair kind, -1: inactive
   const RadialView<R> &T = a.T;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = lane / G, sl = lane % G, gbase = half * G;
+  const int part = SPLIT ? warp : 0, unit = (SPLIT ? 0 : warp * SPW) + half;
   // grid-stride over groups of SPW sites: one group per warp per trip (a full
   // grid makes one trip; a persistent grid of a few blocks per SM makes
   // several); one copy of the body for every trip: a site gives the same
   // bits whichever trip of whichever grid computes it
 #pragma unroll 1
-  for (int wi = blockIdx.x * W + warp; wi * SPW < a.n_real; wi += gridDim.x * W) {
+  for (int wi = SPLIT ? blockIdx.x : blockIdx.x * W + warp; wi * SPW < a.n_real;
+       wi += gridDim.x * (SPLIT ? 1 : W)) {
   const int i = wi * SPW + half;
   const bool live = i < a.n_real && !site_off(a, i);
   const double2 xbi = live ? a.xb[i] : make_double2(0.0, 1.0);
@@ -469,15 +474,15 @@ pass1_kernel(const EvalArgs<R> a) {
   const double4 qi = act ? a.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
   const int ci = act ? a.code[i] : 0;
   const int nb0 = act ? a.offs[i] : 0, nb1 = act ? a.offs[i + 1] : 0;
-  double *site = reinterpret_cast<double *>(&ss[warp * SPW + half]);
-  {  // part I: pair rule, centre and neighbour-displaced points
+  double *site = reinterpret_cast<double *>(&ss[unit]);
+  if (part == 0) {  // part I: pair rule, centre and neighbour-displaced points
     R acc[kP1PartI], lo[kP1PartI];
 #pragma unroll
     for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
 #pragma unroll 1
     for (int p = nb0 + sl; p < nb1; p += G) {
       const NbSite<R> sj = nb_site(a, a.idx[p]);
-      const int c = (warp * SPW + half) * kCap + (p - nb0);  // cache entry
+      const int c = unit * kCap + (p - nb0);  // cache entry
       if (kCap > 0 && p - nb0 < kCap)
         pk_s[c] = sj.active ? (signed char)pair_kind(ci, sj.code) : (signed char)-1;
       if (!sj.active) continue;
@@ -511,6 +516,7 @@ pass1_kernel(const EvalArgs<R> a) {
         site[p1_site_slot(v0 + k)] = tree_total(acc[k], lo[k]);
   }
   if constexpr (sizeof(R) == 4) {  // part II: centre-displaced points
+    if (!SPLIT || part == 1) {
     R acc[kP1PartII], lo[kP1PartII];
 #pragma unroll
     for (int c = 0; c < kP1PartII; ++c) acc[c] = (R)0;
@@ -527,20 +533,22 @@ pass1_kernel(const EvalArgs<R> a) {
     for (int k = 0; k < kP1PartII / G; ++k)
       if (act && t0 + k < 1 + 54)
         site[p1_site_slot(p1_part2_value(t0 + k))] = tree_total(acc[k], lo[k]);
+    }
   } else {
     // FP64: part II one axis at a time (19 live accumulators instead of 55;
     // each displaced point is still evaluated once), sself summed over the
     // three axes in axis order
     double sself = 0.0;
 #pragma unroll 1
-    for (int ax = 0; ax < 3; ++ax) {
+    for (int ax = SPLIT ? part - 1 : 0; ax < (SPLIT ? part : 3); ++ax) {
+      if (SPLIT && part == 0) break;
       R acc[kP1PartI], lo[kP1PartI];
 #pragma unroll
       for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
 #pragma unroll 1
       for (int p = nb0 + sl; p < nb1; p += G) {
         if (kCap > 0 && p - nb0 < kCap) {
-          const int c = (warp * SPW + half) * kCap + (p - nb0);
+          const int c = unit * kCap + (p - nb0);
           const int pk = pk_s[c];
           if (pk < 0) continue;
           const double4 rx = rx_s[c];
@@ -564,19 +572,26 @@ pass1_kernel(const EvalArgs<R> a) {
       }
     }
     // lane 0 of the group held part index 0 in every axis
-    if (act && sl == 0) site[p1_site_slot(kP1Sself)] = sself;
+    if (SPLIT && part > 0 && sl == 0) sself_s[part - 1] = sself;
+    if (!SPLIT && act && sl == 0) site[p1_site_slot(kP1Sself)] = sself;
+  }
+  if constexpr (SPLIT) {
+    __syncthreads();
+    if (sizeof(R) == 8 && act && part == 0 && sl == 0)
+      site[p1_site_slot(kP1Sself)] = (sself_s[0] + sself_s[1]) + sself_s[2];
   }
   __syncwarp();
+  if (part == 0) {
   // epilogue: lanes 0..7 of the group form the record's eight duals, lane 0
   // the rest
   double b = 0.0;
-  if (act && sl < 8) b = site_dual(ss[warp * SPW + half], sl, mom, mom_x<R>(i));
+  if (act && sl < 8) b = site_dual(ss[unit], sl, mom, mom_x<R>(i));
   double bgd = 0.0;
 #pragma unroll
   for (int d = 0; d < 6; ++d) bgd += __shfl_sync(0xffffffffu, b, gbase + 2 + d);
   if (act && sl == 0) {
     SiteResult res;
-    site_scalars(ss[warp * SPW + half], bgd, a.emb[ci], xi, ci, xbi.y, a.gamma[i], qi.w,
+    site_scalars(ss[unit], bgd, a.emb[ci], xi, ci, xbi.y, a.gamma[i], qi.w,
                  a.mass[ci], res, mom, mom_x<R>(i));
     a.rho[i] = res.rho;
     a.V0[i] = res.V0;
@@ -589,7 +604,10 @@ pass1_kernel(const EvalArgs<R> a) {
     for (int c = sl; c < kMomStride; c += G) mom[c] = (R)0;
     if (sl == 0) a.rho[i] = a.V0[i] = a.S0[i] = a.selfx[i] = 0.0;
   }
-  __syncwarp();  // the warp's shared buffers are reused by its next sites
+  }
+  // the shared buffers are reused by the next sites
+  if constexpr (SPLIT) __syncthreads();
+  else __syncwarp();
   }
 }
 
@@ -1302,6 +1320,30 @@ template <class R> void launch_pack(const EvalArgs<R> &a, cudaStream_t st) {
                                                                a.owner, a.s64);
 }
 
+// Undirected pass 1 of a small system, a warp per part of a site, where all its
+// blocks are resident at once, MB an SM (FP64 3 or 4: 444 or 592 sites on 148
+// SMs; FP32C 8: 1,184); beyond, the parts' repeated loads cost more than the
+// shorter chain gives (900 sites in FP64: 34 us in one piece, 52 split).  FP64:
+// 57 sites 13.1 -> 7.6 us, 409 20.3 -> 11.7, 495 21.0 -> 13.2; FP32C: 57 sites
+// 7.1 -> 5.8, 900 15.9 -> 13.8.  Same bits as in one piece.
+template <class R, int MB>
+bool go1_split(const EvalArgs<R> &a, cudaStream_t st, cudaEvent_t mid) {
+  constexpr int W = sizeof(R) == 8 ? 4 : 2;
+  auto k = pass1_kernel<R, W, MB, 32, true, true>;
+  if (smem_grid(k, W * 32, 0, a.n_real) < a.n_real) return false;
+  const int g = a.recs_ready ? 0 : nblocks(a.n_own, 128);
+  if (g > 0) pass1u_pair_kernel<R, 128><<<g, 128, 0, st>>>(a);
+  if (mid) cudaEventRecord(mid, st);
+  k<<<a.n_real, W * 32, 0, st>>>(a);
+  return true;
+}
+template <class R> bool go1_small(const EvalArgs<R> &a, cudaStream_t st, cudaEvent_t mid) {
+  if constexpr (sizeof(R) == 8)
+    return go1_split<R, 3>(a, st, mid) || go1_split<R, 4>(a, st, mid);
+  else
+    return go1_split<R, 8>(a, st, mid);
+}
+
 template <class R>
 cudaError_t launch_pass1(const EvalArgs<R> &a, cudaStream_t st, int v, int v2, cudaEvent_t mid) {
   if (a.n_real <= 0) return cudaSuccess;
@@ -1331,7 +1373,9 @@ cudaError_t launch_pass1(const EvalArgs<R> &a, cudaStream_t st, int v, int v2, c
   case 3: go1<R, 8, 2, 16>(a, st, pers, und, mid); break;
   case 4: go1<R, 4, 5, 16>(a, st, pers, und, mid); break;
   case 5: go1<R, 4, 3, 16>(a, st, pers, und, mid); break;
-  default: go1<R, 4, 1, 32>(a, st, pers, und, mid); break;
+  default:
+    if (!und || pers || !go1_small(a, st, mid)) go1<R, 4, 1, 32>(a, st, pers, und, mid);
+    break;
   }
   return cudaGetLastError();
 }
