@@ -230,6 +230,28 @@ BTAM_HD void ld4(const double *p, double (&v)[4]) {
   for (int c = 0; c < 4; ++c) v[c] = p[c];
 #endif
 }
+// ld4 where `on`, zeros elsewhere, without a branch: the loads around it may
+// be in flight at the same time.
+BTAM_HD void ld4_if(bool on, const float *p, float (&v)[4]) {
+#if defined(__CUDA_ARCH__)
+  v[0] = v[1] = v[2] = v[3] = 0.0f;
+  asm("{ .reg .pred q; setp.ne.s32 q, %5, 0; @q ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4]; }"
+      : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3])
+      : "l"(p), "r"((int)on));
+#else
+  for (int c = 0; c < 4; ++c) v[c] = on ? p[c] : 0.0f;
+#endif
+}
+BTAM_HD void ld4_if(bool on, const double *p, double (&v)[4]) {
+#if defined(__CUDA_ARCH__)
+  v[0] = v[1] = v[2] = v[3] = 0.0;
+  asm("{ .reg .pred q; setp.ne.s32 q, %5, 0; @q ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4]; }"
+      : "+d"(v[0]), "+d"(v[1]), "+d"(v[2]), "+d"(v[3])
+      : "l"(p), "r"((int)on));
+#else
+  for (int c = 0; c < 4; ++c) v[c] = on ? p[c] : 0.0;
+#endif
+}
 // Plain 8-value copy (records staged in shared memory).
 template <class R> BTAM_HD void cp8(const R *p, R (&v)[8]) {
   for (int c = 0; c < 8; ++c) v[c] = p[c];
@@ -440,18 +462,18 @@ BTAM_HD void ld_pr(const RadialView<double> &T, int pk, int m, double (&k)[8]) {
   ld8(pr_rec(T, pk, m), k);
 #endif
 }
-BTAM_HD void ld_pr_h(const RadialView<float> &T, int m, float (&h)[4]) {
+BTAM_HD void ld_pr_h(const RadialView<float> &T, bool on, int m, float (&h)[4]) {
 #if defined(__CUDA_ARCH__)
-  ld4(T.prx + (size_t)16 * T.n + 16 * (size_t)m + 8 * rec64_piece(m, 1), h);
+  ld4_if(on, T.prx + (size_t)16 * T.n + 16 * (size_t)m + 8 * rec64_piece(m, 1), h);
 #else
-  ld4(pr_rec(T, 2, m) + 8, h);
+  ld4_if(on, pr_rec(T, 2, m) + 8, h);
 #endif
 }
-BTAM_HD void ld_pr_h(const RadialView<double> &T, int m, double (&h)[4]) {
+BTAM_HD void ld_pr_h(const RadialView<double> &T, bool on, int m, double (&h)[4]) {
 #if defined(__CUDA_ARCH__)
-  ld4(T.prx + (size_t)16 * (T.n + m) + 4 * rec128_piece(m, 2), h);
+  ld4_if(on, T.prx + (size_t)16 * (T.n + m) + 4 * rec128_piece(m, 2), h);
 #else
-  ld4(pr_rec(T, 2, m) + 8, h);
+  ld4_if(on, pr_rec(T, 2, m) + 8, h);
 #endif
 }
 BTAM_HD void ld_uw(const RadialViewS<float> &T, int pk, int m, float (&k)[8]) {
@@ -489,20 +511,17 @@ BTAM_HD void pr_at(const RadialView<R> &T, int pk, int ci, int cj, int m, R p, R
                    R &rj, R &drj, R &ri, R &dri) {
   R k[8];
   ld_pr(T, pk, m, k);
-  R r0 = (R)0, dr0 = (R)0, r1 = (R)0, dr1 = (R)0;
+  R r0 = (R)0, dr0 = (R)0, r1 = (R)0, dr1 = (R)0, h[4];
+  ld_pr_h(T, pk == 2 && (cj == 1 || (WANT_I && ci == 1)), m, h);
   if (D) {
     cub_vd(k, p, ph, dph);
     cub_vd(k + 4, p, r0, dr0);
+    cub_vd(h, p, r1, dr1);
   } else {
     ph = cub_v(k, p);
     r0 = cub_v(k + 4, p);
+    r1 = cub_v(h, p);
     dph = (R)0;
-  }
-  if (pk == 2 && (cj == 1 || (WANT_I && ci == 1))) {
-    R h[4];
-    ld_pr_h(T, m, h);
-    if (D) cub_vd(h, p, r1, dr1);
-    else r1 = cub_v(h, p);
   }
   const bool jh = pk == 2 && cj == 1, ih = pk == 2 && ci == 1;
   rj = jh ? r1 : r0;

@@ -479,9 +479,11 @@ pass1_kernel(const EvalArgs<R> a) {
     R acc[kP1PartI], lo[kP1PartI];
 #pragma unroll
     for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
+    int jn = nb0 + sl < nb1 ? a.idx[nb0 + sl] : 0;  // the next entry's site, read ahead
 #pragma unroll 1
     for (int p = nb0 + sl; p < nb1; p += G) {
-      const NbSite<R> sj = nb_site(a, a.idx[p]);
+      const NbSite<R> sj = nb_site(a, jn);
+      if (p + G < nb1) jn = a.idx[p + G];
       const int c = unit * kCap + (p - nb0);  // cache entry
       if (kCap > 0 && p - nb0 < kCap)
         pk_s[c] = sj.active ? (signed char)pair_kind(ci, sj.code) : (signed char)-1;
@@ -520,9 +522,11 @@ pass1_kernel(const EvalArgs<R> a) {
     R acc[kP1PartII], lo[kP1PartII];
 #pragma unroll
     for (int c = 0; c < kP1PartII; ++c) acc[c] = (R)0;
+    int jn = nb0 + sl < nb1 ? a.idx[nb0 + sl] : 0;
 #pragma unroll 1
     for (int p = nb0 + sl; p < nb1; p += G) {
-      const NbSite<R> sj = nb_site(a, a.idx[p]);
+      const NbSite<R> sj = nb_site(a, jn);
+      if (p + G < nb1) jn = a.idx[p + G];
       if (!sj.active) continue;
       pass1_pair_part2<R>(T, pair_vec<R>(qi, sj), (R)qi.w, (R)xi * sj.occ,
                           pair_kind(ci, sj.code), acc);
