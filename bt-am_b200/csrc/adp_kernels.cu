@@ -1027,7 +1027,7 @@ template <class R> struct MomShared {
 // occupancy gradient (push_x) into the reverse slot's gx.  What bounds it is
 // the latency and L2-to-SM stream of the kept values, read twice.  38,040-site
 // nanowire (FP32C), per step, before (pass 1 and pass 2 of the undirected
-// kernels) and after: 482 -> 314 us; 2,916-site cell (FP64): 79 -> 33.
+// kernels) and after: 482 -> 294 us; 2,916-site cell (FP64): 79 -> 31.
 template <class R, int W, int MB>
 __global__ void __launch_bounds__(W * 32, MB) kept_site_kernel(const EvalArgs<R> a) {
   constexpr int G = 16, SPW = 2, kOcc = 144;  // slots whose occupancy is cached
@@ -1062,6 +1062,10 @@ __global__ void __launch_bounds__(W * 32, MB) kept_site_kernel(const EvalArgs<R>
       R acc[kP1PartI], lo[kP1PartI];
 #pragma unroll
       for (int c = 0; c < kP1PartI; ++c) acc[c] = (R)0;
+      // the next slot's occupancy and the index after it, read ahead (without: 313 us
+      // a step of the nanowire, 32 of the cell)
+      R xn = nb0 + sl < end ? look(nb0 + sl) : (R)0;
+      int jn = nb0 + sl + G < end ? a.idx[nb0 + sl + G] : 0;
 #pragma unroll 1
       for (int p = nb0 + sl; p < end; p += G) {
         R c0[4], c1[4], c2[4], nb[3][4];
@@ -1070,7 +1074,12 @@ __global__ void __launch_bounds__(W * 32, MB) kept_site_kernel(const EvalArgs<R>
         chunk(2, p, c2);
 #pragma unroll
         for (int k = 0; k < 3; ++k) chunk(6 + k, p, nb[k]);
-        const R xj = look(p);
+        const R xj = xn;
+        if (p + G < end) {
+          const double x = a.xb[jn].x;
+          xn = x < kMinOcc ? (R)-1 : (R)x;
+          if (p + 2 * G < end) jn = a.idx[p + 2 * G];
+        }
         if (p - nb0 < kOcc) occ_c[p - nb0] = xj;
         if (xj < (R)0) continue;
         const R X = xi * xj;
