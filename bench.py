@@ -47,29 +47,27 @@ FLOP_PASS1, FLOP_PASS2 = 1000.0, 2000.0  # algorithmic flops per directed active
 # u, w), 26 at the 13 triplet points (u, w); the algorithmic flops of each
 # pass are attributed to kernels by these lookups
 LOOK_PR, LOOK_TRIP = 48.0, 26.0
-# Per launch of the FP32C kernels on this workload, from one ncu capture
-# (--set full) of the undirected variants (28, 26): DRAM bytes (read +
-# write), and L1 global-load sectors (32 bytes each) with the L1 LSU
-# data-pipe utilisation
-NCU_DRAM_BYTES = {"pass1 pair-rule kernel": 113.1e6, "pass1 site kernel": 65.4e6,
-                  "pass2 pair kernel": 253.2e6, "pass2 site kernel": 75.4e6, "totals": 1.5e6}
+# Per launch of the FP32C kernels on this workload, from one ncu capture of
+# the autotuned variants (27, 30): DRAM bytes (read + write), and L1
+# global-load sectors (32 bytes each) with the L1 LSU data-pipe utilisation
+NCU_DRAM_BYTES = {"pass1 pair-rule kernel": 113.1e6, "pass1 site kernel": 64.1e6,
+                  "pass2 pair kernel": 256.9e6, "pass2 site kernel": 74.9e6, "totals": 1.5e6}
 NCU_L1_SECTORS = {"pass1 pair-rule kernel": 51.73e6, "pass1 site kernel": 54.59e6,
-                  "pass2 pair kernel": 28.55e6, "pass2 site kernel": 2.56e6}
-NCU_L1_PIPE = {"pass1 pair-rule kernel": 0.91, "pass1 site kernel": 0.71,
-               "pass2 pair kernel": 0.69, "pass2 site kernel": 0.31}
+                  "pass2 pair kernel": 52.29e6, "pass2 site kernel": 2.56e6}
+NCU_L1_PIPE = {"pass1 pair-rule kernel": 0.90, "pass1 site kernel": 0.76,
+               "pass2 pair kernel": 0.74, "pass2 site kernel": 0.30}
 # DRAM bytes (read + write) per launch of the FP64 kernels on this workload
-# (autotuned variants (26, 30)), from one ncu capture
-NCU_DRAM_BYTES_FP64 = {"pass1 pair-rule kernel": 264.1e6, "pass1 site kernel": 107.8e6,
-                       "pass2 pair kernel": 486.3e6}
+# (autotuned variants (29, 30)), from one ncu capture
+NCU_DRAM_BYTES_FP64 = {"pass1 pair-rule kernel": 263.3e6, "pass1 site kernel": 105.9e6,
+                       "pass2 pair kernel": 487.4e6}
 # L1 data-pipe wavefront utilisation of the same FP64 launches (ncu
 # l1tex__data_pipe_lsu_wavefronts, share of peak): the binding unit
-NCU_L1_PIPE_FP64 = {"pass1 pair-rule kernel": 0.902, "pass1 site kernel": 0.769,
-                    "pass2 pair kernel": 0.711}
-# shared-memory wavefronts per launch: the pass-2 pair kernel reads its u/w
-# spline records from shared memory (its global sectors are the moment and
-# pair records only)
-NCU_SHARED_WAVEFRONTS = {"pass1 pair-rule kernel": 0.45e6, "pass1 site kernel": 3.35e6,
-                         "pass2 pair kernel": 15.30e6, "pass2 site kernel": 1.37e6}
+NCU_L1_PIPE_FP64 = {"pass1 pair-rule kernel": 0.867, "pass1 site kernel": 0.644,
+                    "pass2 pair kernel": 0.633}
+# shared-memory wavefronts per launch (trees and staged sums; the spline
+# records of these shapes come through L1)
+NCU_SHARED_WAVEFRONTS = {"pass1 pair-rule kernel": 0.77e6, "pass1 site kernel": 4.38e6,
+                         "pass2 pair kernel": 0.51e6, "pass2 site kernel": 1.37e6}
 
 
 def kernel_flops(undirected):
@@ -540,7 +538,7 @@ def bench_bulk_stretch(args, tables, cpu_budget_s=6.0):
            "residual_evaluations": info["evaluations"], "final_norm": info["norm"],
            "status": info["status"], "ms_total": t * 1e3,
            "ms_per_residual": t * 1e3 / max(info["evaluations"], 1),
-           "timing": "host clock around the call (each residual ends in a 96-byte read)"}
+           "timing": "host clock around the call (each residual ends in a 32-byte read)"}
     # the solver the reference's main program configures for this relaxation:
     # N-GMRES(m = 3) with the critical-point line search
     S = btam.System(tables, sys_)
@@ -865,7 +863,7 @@ def run_btam(args, ws, rank, local):
     roofline["l1_data_pipe"] = {
         "bound": "L1 data pipe (random 32-byte halves of the 64-byte FP64 spline records)",
         "ncu_wavefront_frac": NCU_L1_PIPE_FP64,
-        "source": "one ncu capture of the autotuned FP64 shapes (26, 30) on this workload"}
+        "source": "one ncu capture of the autotuned FP64 shapes (29, 30) on this workload"}
     roof32, und32 = kernel_roofline(prof32, shapes["fp32c"], fp32_peak, "fp32", NCU_DRAM_BYTES)
     eval32 = eval_flops / (results["fp32c"]["ms"] * 1e-3) / 1e12
     roof32["evaluation"] = {"flops": eval_flops, "achieved": eval32, "frac": eval32 / fp32_peak,
