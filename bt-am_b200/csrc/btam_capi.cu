@@ -332,6 +332,20 @@ namespace {
 // Doubles from one result array to the next in a system's result block.
 inline size_t result_stride(int n) { return ((size_t)n + 31) & ~(size_t)31; }
 
+// Makes a system's device current for a launch in a call that may come from a
+// thread with another one.
+struct OnDevice {
+  int before = -1;
+  explicit OnDevice(int dev) {
+    int now = dev;
+    if (cudaGetDevice(&now) == cudaSuccess && now != dev && cudaSetDevice(dev) == cudaSuccess)
+      before = now;
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 // Planar q, sigma, x of the sites.
 __global__ void unpack_state_kernel(int n, const double4 *pos, const double2 *xb, double *q,
                                     double *sigma, double *x) {
@@ -361,9 +375,11 @@ struct PinnedRing {
   cudaStream_t st = nullptr;  // copies that pass the system's later kernels
   cudaEvent_t part = nullptr;  // and what they wait for
   unsigned next = 0;           // slots handed out so far
+  // One device a thread, the first; systems of others take plain copies.
   bool ready(int dev) {
-    if (buf && dev == device) return true;
-    release();
+    if (buf) return dev == device;
+    int current = -1;
+    if (cudaGetDevice(&current) != cudaSuccess || current != dev) return false;
     bool ok = cudaHostAlloc(&buf, kSlots * kSlot * sizeof(double), cudaHostAllocDefault) ==
               cudaSuccess;
     for (auto &e : ev)
@@ -2510,6 +2526,7 @@ int btam_dmd_occupancy(btam_system *s, double *x, long long *quanta, double *mu)
   if (!s->dmd_ready) return BTAM_ERR_NOT_BUILT;
   const int n = s->n_real;
   double *dx = s->stage + 4 * (size_t)n, word;
+  const OnDevice on(s->device);
   if (x) {
     unpack_state_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(
         n, s->pos, s->xb, s->stage, s->stage + 3 * (size_t)n, dx);
@@ -2541,6 +2558,7 @@ int btam_system_get_state(btam_system *s, double *q, double *sigma, double *x) {
     BTAM_TRY(cudaStreamSynchronize(s->st));
     return BTAM_OK;
   }
+  const OnDevice on(s->device);
   const int n = s->n_real;
   double *dq = s->stage, *ds = s->stage + 3 * (size_t)n, *dx = s->stage + 4 * (size_t)n;
   unpack_state_kernel<<<(n + 255) / 256, 256, 0, s->st>>>(n, s->pos, s->xb, dq, ds, dx);
