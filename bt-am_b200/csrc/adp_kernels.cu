@@ -1364,7 +1364,7 @@ cudaError_t launch_pass1(const EvalArgs<R> &a, cudaStream_t st, int v, int v2, c
   // the pair-rule records are made (and then also used by pass 1) whenever
   // either pass runs undirected: the undirected pass 2 reads them
   const bool und = ((v | v2) & kUndirected) != 0 && has_undirected(a);
-  if (und && a.x_only && a.kept) {
+  if (takes_kept(a, v2)) {
     if (!a.recs_ready) {
       launch_pack(a, st);
       const int g = nblocks(a.n_own, 128);
@@ -1433,7 +1433,7 @@ template <class R>
 cudaError_t launch_pass2(const EvalArgs<R> &a, cudaStream_t st, int v, cudaEvent_t mid) {
   if (a.n_real <= 0) return cudaSuccess;
   const bool pers = (v & kPersistent) != 0;
-  if ((v & kUndirected) && has_undirected(a) && a.x_only && a.kept) {
+  if (takes_kept(a, v)) {
     if (mid) cudaEventRecord(mid, st);
     auto ks = pass2u_site_kernel<R, 4>;
     ks<<<grid_of(ks, a.n_real, 4, true), 128, 0, st>>>(a);

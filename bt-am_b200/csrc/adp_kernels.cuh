@@ -178,6 +178,12 @@ inline size_t pbuf_values(long long n_slots, long long n_own) {
 template <class R> inline bool has_undirected(const EvalArgs<R> &a) {
   return a.rev && a.pbuf && a.pgx && a.prec1 && a.prec2 && a.slot_own;
 }
+// Whether an evaluation with pass-2 variant v2 runs on the kept values.  Both
+// passes go by this one rule: the kept pass 1 leaves no moment records, which a
+// directed pass 2 would read, whichever form pass 1 itself is pinned to.
+template <class R> inline bool takes_kept(const EvalArgs<R> &a, int v2) {
+  return (v2 & kUndirected) != 0 && has_undirected(a) && a.x_only && a.kept;
+}
 
 // Times every pass-1 and pass-2 variant on this input (reps launches each,
 // synchronising st) and returns the fastest of each.  Every variant computes

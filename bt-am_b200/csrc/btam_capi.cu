@@ -2368,7 +2368,7 @@ DmdArgs dmd_args(btam_system *s) {
 }
 
 // Room for the kept slot values of a run of x-only evaluations (EvalArgs::kept):
-// with undirected variants and a reverse for every entry, if the memory may be
+// with an undirected pass 2 and a reverse for every entry, if the memory may be
 // taken; nullptr else (the evaluations then look everything up each time).
 // Taken from the pool for the call and given back at its end.
 struct KeptSlots {
@@ -2382,7 +2382,7 @@ struct KeptSlots {
     size_t bytes = 0, elem = 0;
     const size_t each = f == 0 ? sizeof(double) : sizeof(float);
     const size_t values = 4 * (size_t)kKeptChunks * (size_t)std::max(s->n_pairs, 1ll);
-    if (((v1 | v2) & kUndirected) && values * each <= s->kept_limit)
+    if ((v2 & kUndirected) && values * each <= s->kept_limit)
       take_pbuf(p, bytes, elem, values, each, s->st);
   }
   ~KeptSlots() { dfree(p, s->st); }

@@ -79,3 +79,33 @@ def test_kept_potentials_equal_the_general_ones(gpu_tables, name, prec):
         xb, Xb, _ = B.dmd_occupancy()
         # a potential's last bits move at most a few quanta's worth of x
         assert np.abs(xa - xb).max() <= 10 * TOL[prec]
+
+
+@pytest.mark.parametrize("control", [False, True])
+@pytest.mark.parametrize("prec", [btam.FP64, btam.FP32C])
+@pytest.mark.parametrize("pair", [(16 | 2, 0), (16, 0 | 8), (0, 16 | 1), (2, 16 | 6 | 8)])
+def test_passes_pinned_to_different_forms(gpu_tables, pair, prec, control):
+    """One pass undirected, the other directed: the potentials are those of the
+    directed kernels at the same state, to the launch-variant test's tolerances
+    (FP64 1e-11, FP32C 1e-5), whatever was evaluated before."""
+    s = cell()
+    S, R = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (S, R):
+        T.build_neighbors()
+    S.set_variants(prec, *pair)
+    R.set_variants(prec, 0, 0)
+    S.evaluate(prec)  # the moments of another state are there
+    S.set_state(sigma=s["sigma"] * 1.1)
+    S.dmd_setup()
+    tol = 1e-11 if prec == btam.FP64 else 1e-5
+    for _ in range(2):
+        x, _, _ = S.dmd_occupancy()
+        R.set_state(sigma=s["sigma"] * 1.1, x=x)
+        want = R.evaluate(prec)["Rx"] + np.where(x < 0.9999, s["gamma"] / s["beta"], 0.0)
+        if control:  # not divided: mu is that of the state x
+            S.dmd_step_ctl(1, prec, max_dx=1.0, max_sub=1, **PRM)
+        else:
+            S.dmd_step(1, prec, **PRM)
+        _, _, mu = S.dmd_occupancy()
+        h = (s["species"] == 1) & (x >= 5e-4)
+        assert np.abs(mu - want)[h].max() <= tol * max(1.0, np.abs(want[h]).max()), pair
