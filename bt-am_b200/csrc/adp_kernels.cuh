@@ -148,6 +148,7 @@ inline void default_variants(bool fp64, int n, int *v1, int *v2) {
 // of the device memory that is free; and not while the stream is being
 // captured (an allocation would belong to the graph).
 bool may_take(size_t need, cudaStream_t st);
+bool capturing(cudaStream_t st);  // or not to be known
 inline bool valid_variants(int v1, int v2) {
   if (v1 < 0 || v2 < 0 || (v1 & ~(2 * kUndirected - 1)) != 0 ||
       (v2 & ~(2 * kUndirected - 1)) != 0)

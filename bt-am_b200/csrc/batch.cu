@@ -215,8 +215,7 @@ void batch_pick_variants(btam_batch *b, int f, int *v1, int *v2) {
   *v2 = b->variant2[f];
   if (*v1 != kAutoVariant) return;
   *v1 = *v2 = kPersistent;
-  if (take_pbuf(b->pbuf, b->pbuf_bytes, b->pbuf_elem,
-                pbuf_values(b->n_pairs > 0 ? b->n_pairs : 1, b->n_own),
+  if (take_pbuf(b->pbuf, b->pbuf_bytes, pbuf_values(b->n_pairs > 0 ? b->n_pairs : 1, b->n_own),
                 f == 0 ? sizeof(double) : sizeof(float), b->st)) {
     default_variants(f == 0, b->n_real, v1, v2);
     *v1 |= kPersistent;

@@ -291,6 +291,23 @@ template <class R> EvalArgs<R> eval_args(btam_system *s, R *mom, const RadialVie
   return a;
 }
 
+// Gives the pair buffer up: back to the pool, or kept aside for a captured
+// evaluation that writes to it.
+void drop_pbuf(btam_system *s) {
+  if (s->pbuf && s->pbuf_captured) {
+    s->pbuf_old.push_back(s->pbuf);
+    s->pbuf = nullptr;
+  }
+  dfree(s->pbuf, s->st);
+  s->pbuf_bytes = 0;
+}
+// The buffers kept aside go when no captured evaluation can use them any more.
+void drop_old_pbufs(btam_system *s) {
+  for (char *&p : s->pbuf_old) dfree(p, s->st);
+  s->pbuf_old.clear();
+  s->pbuf_captured = false;
+}
+
 // Buffer of the undirected kernels, allocated only when an undirected variant
 // is in use: the pass-2 slot records of the real sites' lists (5 values of R
 // per slot), then the pair-rule records of the owned pairs (prec1, prec2);
@@ -301,7 +318,7 @@ int ensure_pbuf(btam_system *s, size_t elem) {
       pbuf_values(s->n_pairs > 0 ? s->n_pairs : 1, s->n_own) * elem;
   s->pbuf_elem = elem;
   if (need <= s->pbuf_bytes) return BTAM_OK;
-  s->pbuf_bytes = 0;
+  drop_pbuf(s);
   BTAM_TRY(dalloc(s->pbuf, s->st, need));
   s->pbuf_bytes = need;
   return BTAM_OK;
@@ -310,14 +327,20 @@ int ensure_pbuf(btam_system *s, size_t elem) {
 // The launch variants of the system's next evaluation in form f (0 FP64, 1
 // FP32C): the pinned or tuned ones, else default_variants if their pair
 // buffer is there or may be taken, else the directed kernels, which need none.
+// A captured evaluation of the defaults is directed, whatever is there: its
+// graph outlives the buffer that the defaults take and give up as they need.
 void pick_variants(btam_system *s, int f, int *v1, int *v2) {
   *v1 = s->variant1[f];
   *v2 = s->variant2[f];
-  if (*v1 != kAutoVariant) return;
+  if (*v1 != kAutoVariant) {
+    if (((*v1 | *v2) & kUndirected) && !s->pbuf_captured) s->pbuf_captured = capturing(s->st);
+    return;
+  }
   *v1 = *v2 = 0;
-  const size_t elem = f == 0 ? sizeof(double) : sizeof(float);
-  if (take_pbuf(s->pbuf, s->pbuf_bytes, s->pbuf_elem,
-                pbuf_values(s->n_pairs > 0 ? s->n_pairs : 1, s->n_own), elem, s->st))
+  if (capturing(s->st)) return;
+  if (take_pbuf(s->pbuf, s->pbuf_bytes, pbuf_values(s->n_pairs > 0 ? s->n_pairs : 1, s->n_own),
+                f == 0 ? sizeof(double) : sizeof(float), s->st,
+                s->pbuf_captured ? &s->pbuf_old : nullptr))
     default_variants(f == 0, s->n_real, v1, v2);
 }
 
@@ -645,12 +668,15 @@ cudaMemPool_t device_pool() {
   return pools[dev];
 }
 
-bool may_take(size_t need, cudaStream_t st) {
+bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return false;
-  }
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
+bool may_take(size_t need, cudaStream_t st) {
+  if (capturing(st)) return false;
   cudaMemPool_t pool = device_pool();
   unsigned long long used = 0, held = 0;
   size_t spare = 0;
@@ -997,6 +1023,7 @@ void btam_system_destroy(btam_system *s) {
   dfree(s->dact, s->st); dfree(s->dout, s->st); dfree(s->din, s->st); dfree(s->rv, s->st);
   dfree(s->rev, s->st); dfree(s->slot_own, s->st); dfree(s->own_off, s->st); dfree(s->own_p, s->st); dfree(s->own_u, s->st);
   dfree(s->pbuf, s->st);
+  drop_old_pbufs(s);
   s->scratch.release(s->st);
   if (s->st) cudaStreamSynchronize(s->st);
   if (s->st) cudaStreamDestroy(s->st);
@@ -1111,6 +1138,7 @@ int btam_neighbors_build(btam_system *s, int all_sites) {
   BTAM_TRY(launch_pair_links(n, s->offs, s->idx, s->owner, s->rev, s->slot_own, s->cnt,
                              s->own_off, s->own_p, s->own_u, s->own_cap, &s->n_own, &s->n_unpaired,
                              s->scratch, s->st));
+  drop_old_pbufs(s);  // captured evaluations are of the lists that were
   // a rebuilt list may be longer than the pair buffer: pinned undirected
   // variants need it, the defaults take it again at the next evaluation
   bool pinned = false;
@@ -1263,8 +1291,8 @@ int btam_autotune(btam_system *s, int precision, int *pass1_variant, int *pass2_
   if (st != BTAM_OK) return st;
   // the slot buffer stays only while an undirected variant is selected
   if (!((s->variant1[0] | s->variant1[1] | s->variant2[0] | s->variant2[1]) & kUndirected)) {
-    dfree(s->pbuf, s->st);
-    s->pbuf_bytes = s->pbuf_elem = 0;
+    drop_pbuf(s);
+    s->pbuf_elem = 0;
   }
   const int f = precision == BTAM_FP64 ? 0 : 1;
   if (pass1_variant) *pass1_variant = s->variant1[f];
@@ -2379,11 +2407,11 @@ struct KeptSlots {
     int v1 = 0, v2 = 0;
     if (nsteps <= 0 || !s->built || s->batcher || s->n_unpaired > 0 || s->n_list != s->n_real) return;
     pick_variants(s, f, &v1, &v2);
-    size_t bytes = 0, elem = 0;
+    size_t bytes = 0;
     const size_t each = f == 0 ? sizeof(double) : sizeof(float);
     const size_t values = 4 * (size_t)kKeptChunks * (size_t)std::max(s->n_pairs, 1ll);
     if ((v2 & kUndirected) && values * each <= s->kept_limit)
-      take_pbuf(p, bytes, elem, values, each, s->st);
+      take_pbuf(p, bytes, values, each, s->st);
   }
   ~KeptSlots() { dfree(p, s->st); }
 };

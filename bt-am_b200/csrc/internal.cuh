@@ -100,7 +100,11 @@ struct btam_system {
   // most bytes a master-equation call may take for kept slot values
   size_t kept_limit = (size_t)-1;
   char *pbuf = nullptr;
-  size_t pbuf_bytes = 0, pbuf_elem = 0;  // bytes; bytes per value (0: none yet)
+  size_t pbuf_bytes = 0, pbuf_elem = 0;  // bytes; bytes per value of pinned forms
+  // a captured evaluation writes to pbuf: a larger one then leaves it in place,
+  // in pbuf_old, until the lists are rebuilt or the system ends
+  bool pbuf_captured = false;
+  std::vector<char *> pbuf_old;
   // non-mean-field forms: site records, outputs and totals (point.cu)
   double *pt = nullptr;
   size_t pt_cap = 0;
@@ -241,25 +245,24 @@ template <class T> inline void dfree(T *&p, cudaStream_t st) {
   p = nullptr;
 }
 
-// Pair buffer for the default variants: `values` values of at least `elem`
-// bytes, if they are there or may be taken (may_take).  The buffer that is
-// there stays when they are not.
-inline bool take_pbuf(char *&pbuf, size_t &bytes, size_t &held_elem, size_t values, size_t elem,
-                      cudaStream_t st) {
-  if (elem < held_elem) elem = held_elem;
+// Pair buffer for the default variants: `values` values of `elem` bytes, if
+// they are there or may be taken (may_take).  The buffer that is there stays
+// when they are not; a smaller one goes to `old`, or back to the pool if that
+// is null.
+inline bool take_pbuf(char *&pbuf, size_t &bytes, size_t values, size_t elem, cudaStream_t st,
+                      std::vector<char *> *old = nullptr) {
   const size_t need = values * elem;
-  if (need > bytes) {
-    char *p = nullptr;
-    if (!may_take(need, st)) return false;
-    if (dalloc(p, st, need) != cudaSuccess) {
-      cudaGetLastError();  // nothing is left to report: other kernels run
-      return false;
-    }
-    dfree(pbuf, st);
-    pbuf = p;
-    bytes = need;
+  if (need <= bytes) return true;
+  char *p = nullptr;
+  if (!may_take(need, st)) return false;
+  if (dalloc(p, st, need) != cudaSuccess) {
+    cudaGetLastError();  // nothing is left to report: other kernels run
+    return false;
   }
-  held_elem = elem;
+  if (old && pbuf) old->push_back(pbuf);
+  else dfree(pbuf, st);
+  pbuf = p;
+  bytes = need;
   return true;
 }
 

@@ -265,8 +265,12 @@ int btam_system_sync(btam_system *s);
  * the last bits (within the stated tolerance of the form).  A system (or
  * batch) that is neither tuned nor pinned takes undirected shapes by its
  * size, or the directed kernels (0, 0) where their pair buffer would be more
- * than 256 MB and more than a quarter of the free device memory, cannot be
- * had, or would have to be allocated inside a stream capture. */
+ * than 256 MB and more than a quarter of the free device memory, or cannot be
+ * had.  Under stream capture such a system takes the directed kernels, which
+ * need no buffer; pin its variants for a captured evaluation that gives the
+ * bits of the uncaptured one.  A captured evaluation may be replayed until the
+ * system's lists are rebuilt or the system is destroyed, whatever else is
+ * evaluated, tuned or pinned in between. */
 int btam_autotune(btam_system *s, int precision, int *pass1_variant, int *pass2_variant);
 /* Pins the launch variants of `precision` (as reported by btam_autotune),
  * for runs that must reproduce one another bit for bit. */
