@@ -2416,6 +2416,19 @@ struct KeptSlots {
   ~KeptSlots() { dfree(p, s->st); }
 };
 
+// Full residuals of the state that the last step of a call moves from, for a
+// system left to the defaults, which any evaluation leaves with them; between
+// the step's chemical potentials, which do not change with the number of steps
+// in a call, and its moves.  (Directed kernels and served rounds have already
+// formed them.)
+int dmd_residuals(btam_system *s, int precision) {
+  const int f = precision == BTAM_FP64 ? 0 : 1;
+  if (s->batcher || s->variant1[f] != kAutoVariant) return BTAM_OK;
+  int v1 = 0, v2 = 0;
+  pick_variants(s, f, &v1, &v2);
+  return (v2 & kUndirected) ? enqueue_eval(s, precision, false, false, false) : BTAM_OK;
+}
+
 int dmd_finish(btam_system *s, long long *total_quanta) {
   if (total_quanta) {
     BTAM_TRY(dmd_total(s->n_real, s->code, s->X, s->dtot, s->st));
@@ -2443,7 +2456,9 @@ int btam_dmd_step(btam_system *s, int precision, int nsteps, const double *param
     // move during the steps, so what depends on them alone is kept
     int st = enqueue_eval(s, precision, true, k > 0, false, kept.p);
     if (st != BTAM_OK) return st;
-    BTAM_TRY(dmd_step(a, prm, s->st));
+    BTAM_TRY(dmd_prepare(a, prm, s->st));
+    if (k == nsteps - 1 && (st = dmd_residuals(s, precision)) != BTAM_OK) return st;
+    BTAM_TRY(dmd_apply(a, prm, s->st));
   }
   if (nsteps > 0) {
     int st = relax_totals(s);
@@ -2452,8 +2467,12 @@ int btam_dmd_step(btam_system *s, int precision, int nsteps, const double *param
   return dmd_finish(s, total_quanta);
 }
 
-int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *params,
-                      long long *total_quanta, double *stats) {
+}  // extern "C"
+
+// btam_dmd_step_ctl; residuals: dmd_residuals in the last sub-step (a caller
+// that evaluates in full right after the steps needs none).
+static int dmd_controlled(btam_system *s, int precision, int nsteps, const double *params,
+                          bool residuals, long long *total_quanta, double *stats) {
   if (!s || nsteps < 0) return BTAM_ERR_ARG;
   if (!s->dmd_ready) return BTAM_ERR_NOT_BUILT;
   DmdParams prm;
@@ -2491,6 +2510,9 @@ int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *p
         if ((st = enqueue_eval(s, precision, true, true, false, kept.p)) != BTAM_OK) return st;
         BTAM_TRY(dmd_prepare(a, prm, s->st));
       }
+      if (residuals && k == nsteps - 1 && j == m - 1 &&
+          (st = dmd_residuals(s, precision)) != BTAM_OK)
+        return st;
       BTAM_TRY(dmd_apply(a, sub, s->st));
     }
     subs += m;
@@ -2509,6 +2531,13 @@ int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *p
   return st;
 }
 
+extern "C" {
+
+int btam_dmd_step_ctl(btam_system *s, int precision, int nsteps, const double *params,
+                      long long *total_quanta, double *stats) {
+  return dmd_controlled(s, precision, nsteps, params, true, total_quanta, stats);
+}
+
 int btam_dmd_run(btam_system *s, int precision, int nsteps, const double *params,
                  int relax_every, int relax_mode, double relax_tol, int relax_max_iter,
                  long long *total_quanta, double *stats) {
@@ -2519,12 +2548,13 @@ int btam_dmd_run(btam_system *s, int precision, int nsteps, const double *params
   while (done < nsteps) {
     const int k = relax_every > 0 ? std::min(relax_every, nsteps - done) : nsteps - done;
     double st4[4] = {0, 0, 0, 0};
-    int st = btam_dmd_step_ctl(s, precision, k, params, nullptr, st4);
+    const bool relax = relax_every > 0 && (done + k) % relax_every == 0;
+    int st = dmd_controlled(s, precision, k, params, !relax, nullptr, st4);
     if (st != BTAM_OK) return st;
     for (int c = 0; c < 3; ++c) acc[c] += st4[c];
     acc[3] = std::max(acc[3], st4[3]);
     done += k;
-    if (relax_every > 0 && done % relax_every == 0) {
+    if (relax) {
       // the mechanical state follows the new occupancies
       double info[5] = {0, 0, 0, 0, 0};
       st = btam_relax(s, relax_mode, relax_tol, relax_max_iter,

@@ -640,11 +640,6 @@ cudaError_t dmd_apply(const DmdArgs &a, const DmdParams &prm, cudaStream_t st) {
   return dmd_commit(a, st);
 }
 
-cudaError_t dmd_step(const DmdArgs &a, const DmdParams &prm, cudaStream_t st) {
-  cudaError_t e = dmd_prepare(a, prm, st);
-  return e == cudaSuccess ? dmd_apply(a, prm, st) : e;
-}
-
 cudaError_t dmd_total(int n, const int *code, const long long *X, long long *out2,
                       cudaStream_t st) {
   dmd_total_kernel<<<1, 1024, 0, st>>>(n, code, X, out2);

@@ -89,8 +89,7 @@ struct DmdArgs {
 cudaError_t dmd_init(int n, const double2 *xb, const int *code, long long *X, cudaStream_t st);
 // x of every H site and image from the quanta, which become the snapshot.
 cudaError_t dmd_commit(const DmdArgs &a, cudaStream_t st);
-cudaError_t dmd_step(const DmdArgs &a, const DmdParams &prm, cudaStream_t st);
-// The step in its parts: chemical potentials, activity and rooms of the
+// A step in its parts: chemical potentials, activity and rooms of the
 // current state; then (optionally) the step-control decision for a step
 // of prm.dt into ctl[0..1]; then the occupancy update of one step of
 // prm.dt (edge moves, commit).

@@ -109,3 +109,39 @@ def test_passes_pinned_to_different_forms(gpu_tables, pair, prec, control):
         _, _, mu = S.dmd_occupancy()
         h = (s["species"] == 1) & (x >= 5e-4)
         assert np.abs(mu - want)[h].max() <= tol * max(1.0, np.abs(want[h]).max()), pair
+
+
+@pytest.mark.parametrize("sub", [0, 1, 4])
+@pytest.mark.parametrize("prec", [btam.FP64, btam.FP32C])
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_default_systems_keep_full_residuals(gpu_tables, name, prec, sub):
+    """Neither tuned nor pinned: the steps leave the full evaluation of the state
+    that the last (sub-)step moved from, bit for bit (the same default kernels),
+    and move as the same steps one at a time.  sub 0: plain steps; else controlled
+    ones of at most `sub` sub-steps."""
+    s = SYSTEMS[name]()
+    S, R = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (S, R):
+        T.build_neighbors()
+        T.dmd_setup()
+    for nsteps in (3, 1):
+        m = 1
+        if sub:
+            total, st = S.dmd_step_ctl(nsteps, prec, max_dx=1e-6, max_sub=sub, **PRM)
+            m = st["substeps"] // nsteps
+            assert m == sub
+        else:
+            total = S.dmd_step(nsteps, prec, **PRM)
+        part = dict(PRM, dt=PRM["dt"] / m)
+        for k in range(nsteps * m - 1):
+            R.dmd_step(1, prec, **part)
+        E = btam.System(gpu_tables, s)
+        E.build_neighbors()
+        E.set_state(x=R.dmd_occupancy()[0])
+        want = E.evaluate(prec)
+        got = S.results(want=tuple(want))
+        for k, v in want.items():
+            assert np.array_equal(got[k], v), (name, k)
+        assert np.any(got["Rq"]) and got["totals"][2] > 0.0
+        assert R.dmd_step(1, prec, **part) == total
+        assert np.array_equal(S.dmd_occupancy()[1], R.dmd_occupancy()[1])
