@@ -280,6 +280,7 @@ __device__ __forceinline__ void pt_entries(const PtArgs &a, const V3<double> &F,
     double pp, dph, rj, drj;
     const int m = geo_uw<double, true>(g, e[k].r, a.T, pk, pp);
     pr_slopes(a.T, pk, cj[k], m, pp, dph, rj, drj);
+    if (x == 0.0) g.inv_s = 0.0;  // an empty site may lie at u itself
     e[k].A = x * drj * g.inv_s;
     e[k].B = 0.5 * (t * dph) * g.inv_s;
     e[k].tu = t * g.u;

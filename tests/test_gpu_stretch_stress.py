@@ -46,3 +46,24 @@ def test_residual_equals_the_point_forms_stress(gpu_tables, name, F0):
     W = S.pt_eval()["W"]
     d = np.stack([W[:, a, a] for a in range(3)], 1) / (np.array(F0) * info["volume"])
     assert abs(info["norm"] - np.linalg.norm(d.sum(0))) <= 1e-11 * np.abs(d).sum()
+
+
+@pytest.mark.parametrize("x", [0.0, 1e-4])
+@pytest.mark.parametrize("name", ["cell", "full_cell", "sphere"])
+def test_empty_sites_at_occupied_ones(gpu_tables, name, x):
+    """An empty site at exactly the position of an occupied one weighs nothing in
+    the residual, as in the point forms: same tolerance, nothing not finite."""
+    s = SYSTEMS[name]()
+    at = np.flatnonzero(s["x"] > 0.1)[::7]
+    n = len(at)
+    s = dict(s, q=np.vstack([s["q"], s["q"][at]]), sigma=np.append(s["sigma"], s["sigma"][at]),
+             x=np.append(s["x"], np.full(n, x)),
+             species=np.append(s["species"], np.ones(n, s["species"].dtype)),
+             beta=np.append(s["beta"], s["beta"][at]), gamma=np.append(s["gamma"], np.zeros(n)))
+    S = btam.System(gpu_tables, s)
+    S.build_neighbors()
+    F0 = (0.985, 1.01, 1.02)
+    _, info = S.relax_stretch(max_iter=0, F0=F0)
+    W = S.pt_eval()["W"]
+    d = np.stack([W[:, a, a] for a in range(3)], 1) / (np.array(F0) * info["volume"])
+    assert abs(info["norm"] - np.linalg.norm(d.sum(0))) <= 1e-11 * np.abs(d).sum()
