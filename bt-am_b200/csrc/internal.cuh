@@ -97,8 +97,13 @@ struct btam_system {
   int n_unpaired = 0;      // entries without a reverse (rev < 0)
   bool same_beta = false;  // every site has the same beta
   bool served = false;  // a server's job
-  // most bytes a master-equation call may take for kept slot values
-  size_t kept_limit = (size_t)-1;
+  // most bytes a master-equation call may take for kept slot values: they go
+  // back to the library's pool, which returns nothing to the device by itself,
+  // and taking them from the device costs 10 to 30 ms a GB once.  4 GB is 2 % of
+  // the device; larger systems look everything up in each evaluation (120,960
+  // sites in FP64: 3.7 ms a step against 2.1 with kept values)
+  static constexpr size_t kKeptMost = (size_t)4 << 30;
+  size_t kept_limit = kKeptMost;
   char *pbuf = nullptr;
   size_t pbuf_bytes = 0, pbuf_elem = 0;  // bytes; bytes per value of pinned forms
   // a captured evaluation writes to pbuf: a larger one then leaves it in place,

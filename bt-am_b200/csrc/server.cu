@@ -323,7 +323,7 @@ void run_job(btam_server *srv, Job *job) {
     // kept slot values only within what admission counted for the job's lists
     const size_t counted = (size_t)n * BTAM_MAXNEIGH * kSlotBytes;
     const size_t used = (size_t)s->n_pairs * 8 + s->pbuf_bytes + (size_t)s->n_own * 8;
-    s->kept_limit = counted > used ? counted - used : 0;
+    s->kept_limit = std::min(counted > used ? counted - used : 0, btam_system::kKeptMost);
   } else if (st == BTAM_OK) {  // the plain two-pass pair
     st = btam_set_variants(s, BTAM_FP32C, 0, 0);
     if (st == BTAM_OK) st = btam_set_variants(s, BTAM_FP64, 0, 0);

@@ -519,6 +519,11 @@ int btam_relax_newton(btam_system *s, double tol, int max_newton, int max_cg,
  *   dt * Df/dr^2 * (beta_i+beta_j)/2 * xm(1-xm) * (mu_i - mu_j),  xm = (x_i+x_j)/2,
  * rounded to quanta, skipped below min_dx, limited so that no site leaves
  * [0, max(max_x, x)], from i to j.  Total hydrogen is conserved exactly.
+ * While a call runs, undirected variants hold 36 values per entry of the
+ * neighbour lists, from the library's memory pool (which keeps what it has
+ * taken for later systems): at most 4 GB, and within the limits of the default
+ * variants' pair buffer (btam_autotune).  Beyond, each evaluation looks
+ * everything up.
  * params (5, NULL = reference values): dt (4e-4), Df (0.045), dr (3.2),
  * min_dx (1e-8), max_x (0.9).  total_quanta (2, may be NULL): 128-bit total
  * of the quanta after the steps, as (high, low) 64-bit halves. */

@@ -145,3 +145,26 @@ def test_default_systems_keep_full_residuals(gpu_tables, name, prec, sub):
         assert np.any(got["Rq"]) and got["totals"][2] > 0.0
         assert R.dmd_step(1, prec, **part) == total
         assert np.array_equal(S.dmd_occupancy()[1], R.dmd_occupancy()[1])
+
+
+def test_kept_values_are_bounded(gpu_tables):
+    """Steps of a system whose kept values would exceed 4 GB leave no more than
+    their small arrays in the library's pool (256 MB), and move as the general
+    evaluation says (the x-only test's tolerance)."""
+    torch = pytest.importorskip("torch")
+    s = lattice.supercell(30, 28, 24, h_fraction=1.0, x_range=(0.1, 0.6), seed=24)
+    S = btam.System(gpu_tables, s)
+    S.build_neighbors()
+    S.set_variants(btam.FP64, 16 | 5, 16 | 6)
+    ref = S.evaluate_x(btam.FP64)["Rx"] + s["gamma"] / s["beta"]
+    S.dmd_setup()
+    assert S.neighbors()[1].size * 36 * 8 > (4 << 30)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    S.dmd_step(1, btam.FP64, **dict(PRM, dt=0.0))
+    h = s["species"] == 1
+    mu = S.dmd_occupancy()[2][h]
+    assert np.abs(mu - ref[h]).max() <= TOL[btam.FP64] * max(1.0, np.abs(ref[h]).max())
+    S.dmd_step(2, btam.FP64, **PRM)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= 256 << 20
