@@ -16,6 +16,7 @@
 
 #include "../../include/btam.h"
 #include "adp_core.cuh"
+#include "idle_list.hpp"
 #include "linalg.hpp"
 #include "adp_kernels.cuh"
 #include "solvers.cuh"
@@ -383,13 +384,12 @@ __global__ void unpack_state_kernel(int n, const double4 *pos, const double2 *xb
 }
 
 // Pinned buffers of the calling thread for copies between a system's arrays and
-// the caller's pageable ones: 1 MB in four slots, made by the first such copy and
-// freed with the thread.  A cudaMemcpyAsync on pageable memory costs some 8 us
-// of calls and waits beside its bytes, so what fits one slot moves as one block;
-// larger results pass through the slots, the copy engine filling one while the
-// host empties another (27,000 sites' results: 216 -> 139 us).  Inputs larger
-// than a slot are as fast without it (106 us against 121).
-struct PinnedRing {
+// the caller's pageable ones: 1 MB in four slots.  A cudaMemcpyAsync on pageable
+// memory costs some 8 us of calls and waits beside its bytes, so what fits one
+// slot moves as one block; larger results pass through the slots, the copy engine
+// filling one while the host empties another (27,000 sites' results: 216 -> 139
+// us).  Inputs larger than a slot are as fast without it (106 us against 121).
+struct RingParts {
   static constexpr int kSlots = 4;
   static constexpr size_t kSlot = 32768;  // doubles
   int device = -1;
@@ -398,11 +398,7 @@ struct PinnedRing {
   cudaStream_t st = nullptr;  // copies that pass the system's later kernels
   cudaEvent_t part = nullptr;  // and what they wait for
   unsigned next = 0;           // slots handed out so far
-  // One device a thread, the first; systems of others take plain copies.
-  bool ready(int dev) {
-    if (buf) return dev == device;
-    int current = -1;
-    if (cudaGetDevice(&current) != cudaSuccess || current != dev) return false;
+  bool make(int dev) {
     bool ok = cudaHostAlloc(&buf, kSlots * kSlot * sizeof(double), cudaHostAllocDefault) ==
               cudaSuccess;
     for (auto &e : ev)
@@ -423,17 +419,34 @@ struct PinnedRing {
     if (part) cudaEventDestroy(part);
     if (st) cudaStreamDestroy(st);
     if (buf) cudaFreeHost(buf);
-    buf = nullptr;
-    part = nullptr;
-    st = nullptr;
-    for (auto &e : ev) e = nullptr;
-    device = -1;
+    *this = RingParts();
+  }
+};
+
+// Rings of threads that have ended, for the next ones.  Never destroyed: threads
+// may end after the statics of the process.
+IdleList<RingParts> &idle_rings() {
+  static IdleList<RingParts> *r = new IdleList<RingParts>;
+  return *r;
+}
+void free_ring(RingParts &r) { r.release(); }
+
+struct PinnedRing : RingParts {
+  int asked = 0;  // two to four times a call
+  // One device a thread, the first; systems of others take plain copies.
+  bool ready(int dev) {
+    if (buf) return dev == device;
+    int current = -1;
+    if (cudaGetDevice(&current) != cudaSuccess || current != dev) return false;
+    return idle_rings().acquire(dev, asked, *this, [dev](RingParts &r) { return r.make(dev); });
   }
   // slot k may still be the source of another stream's copy: wait for its event
   // before writing it (one that was never recorded counts as completed)
   double *slot(unsigned k) { return buf + (k % kSlots) * kSlot; }
   cudaEvent_t event(unsigned k) { return ev[k % kSlots]; }
-  ~PinnedRing() { release(); }
+  ~PinnedRing() {
+    if (buf) idle_rings().leave(*this, free_ring);
+  }
 };
 thread_local PinnedRing pinned_ring;
 
@@ -758,6 +771,7 @@ int btam_tables_load(const char *dir, btam_tables **out) {
     delete t;
     return BTAM_ERR_IO;
   }
+  idle_rings().users(1, free_ring);
   cudaGetDevice(&t->device);
   size_t total = 0;
   for (int k = 0; k < T_COUNT; ++k) total += t->host.t[k].n;
@@ -891,6 +905,7 @@ void btam_tables_destroy(btam_tables *t) {
   if (t->uws32) cudaFree(t->uws32);
   if (t->uws64) cudaFree(t->uws64);
   delete t;
+  idle_rings().users(-1, free_ring);
 }
 
 double btam_tables_mass(const btam_tables *t, int species) {

@@ -82,3 +82,33 @@ def test_systems_of_one_thread_share_the_slots(gpu_tables):
             S.set_state(sigma=s["sigma"] * (1.0 + 0.01 * (r + k)))
         for k, (S, s) in enumerate(pairs):
             assert np.array_equal(S.get_state()[1], s["sigma"] * (1.0 + 0.01 * (r + k)))
+
+
+def test_threads_that_end_hand_their_slots_on(gpu_tables):
+    """Jobs on threads of their own, eight at a time, each with more copies than a
+    thread waits for slots of its own: the bits of one thread's."""
+    dicts = [lattice.sphere(9.0 + k % 7, h_fraction=0.3, seed=k) for k in range(48)]
+    bad = []
+
+    def job(k, ref):
+        S = btam.System(gpu_tables, dicts[k])
+        S.build_neighbors()
+        for r in range(1 + 15 * (k % 3)):
+            sigma = np.asarray(dicts[k]["sigma"]) * (1.0 + 0.01 * r)
+            o = S.evaluate_state(btam.FP64, sigma=sigma)
+            if not np.array_equal(S.get_state()[1], sigma):
+                bad.append(k)
+            if ref is not None and r == 0:
+                bad.extend(k for c in KEYS if not np.array_equal(o[c], ref[c]))
+            if r == 0:
+                first = o
+        return first
+
+    ref = [job(k, None) for k in range(len(dicts))]
+    for a in range(0, len(dicts), 8):
+        ts = [threading.Thread(target=job, args=(k, ref[k])) for k in range(a, a + 8)]
+        for x in ts:
+            x.start()
+        for x in ts:
+            x.join()
+    assert not bad
