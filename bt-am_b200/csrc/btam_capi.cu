@@ -1822,6 +1822,14 @@ cudaError_t relax_move(btam_system *s, const RelaxVecs &v, const double *z0, con
                      s->st);
 }
 
+// The totals of the last evaluation (a served one brought its own).
+int relax_totals(btam_system *s) {
+  if (s->batcher) return BTAM_OK;
+  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->tot_part,
+                         s->st));
+  return BTAM_OK;
+}
+
 // Evaluation of the state and the relaxation's view of it (z, g), with one
 // wait for its scalars: F, |R|^2 and the error bits, and (step) lbfgs_step's.
 int relax_eval(btam_system *s, int prec, RelaxVecs &v, double &f, double &r2,
@@ -1836,15 +1844,10 @@ int relax_eval(btam_system *s, int prec, RelaxVecs &v, double &f, double &r2,
     for (int c = 0; c < 4; ++c) step[c] = h[c];
   f = h[4];
   r2 = h[5];
-  return status_from_bits((int)h[6]);
-}
-
-// The totals of the last evaluation (a served one brought its own).
-int relax_totals(btam_system *s) {
-  if (s->batcher) return BTAM_OK;
-  BTAM_TRY(launch_totals(s->n_real, s->V0, s->S0, s->Rq, s->Rs, s->Rx, s->totals, s->tot_part,
-                         s->st));
-  return BTAM_OK;
+  const int bad = status_from_bits((int)h[6]);
+  if (bad == BTAM_OK) return BTAM_OK;
+  st = relax_totals(s);  // the relaxation ends here, its results stay complete
+  return st == BTAM_OK ? bad : st;
 }
 
 double dev_dot(btam_system *s, RelaxVecs &v, int n, const double *a, const double *b) {

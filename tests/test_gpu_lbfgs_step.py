@@ -108,3 +108,27 @@ def test_relaxation_iterates(gpu_tables, make, m):
     assert abs(info["objective"] - want_F) <= 1e-10 * abs(want_F)
     # the totals left behind are those of the final state, images included
     assert np.array_equal(S.results(want=("totals",))["totals"], S.evaluate()["totals"])
+
+
+@pytest.mark.parametrize("relax", [dict(mode=btam.RELAX_FP64), dict(mode=btam.RELAX_MIXED)],
+                         ids=["fp64", "mixed"])
+def test_totals_of_a_failed_relaxation(gpu_tables, relax):
+    """An evaluation that is not finite (two occupied sites at one position) ends
+    the relaxation with its error and leaves that evaluation's results, the
+    totals among them."""
+    s = open_sphere()
+    h = np.flatnonzero((s["species"] == 1) & (s["x"] > 0.1))
+    s["q"][h[1]] = s["q"][h[0]]
+    prec = btam.FP64 if relax["mode"] == btam.RELAX_FP64 else btam.FP32C
+    S, R = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (S, R):
+        T.build_neighbors()
+    with pytest.raises(btam.BtamError) as want:
+        R.evaluate(prec)
+    with pytest.raises(btam.BtamError) as got:
+        S.relax(tol=1e-8, max_iter=3, **relax)
+    assert got.value.code == want.value.code == 6  # BTAM_ERR_NONFINITE
+    keys = ("rho", "V0", "S0", "Rq", "Rs", "Rx", "totals")
+    a, b = S.results(want=keys), R.results(want=keys)
+    for k in keys:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
