@@ -2518,7 +2518,11 @@ static int dmd_controlled(btam_system *s, int precision, int nsteps, const doubl
     double r[2];
     std::memcpy(r, bits, sizeof(r));
     const double need = std::max(r[0], r[1]);
-    if (!std::isfinite(need)) return BTAM_ERR_NONFINITE;
+    if (!std::isfinite(need)) {  // the call ends here, the results stay complete
+      st = residuals ? dmd_residuals(s, precision) : BTAM_OK;
+      if (st == BTAM_OK) st = relax_totals(s);
+      return st == BTAM_OK ? BTAM_ERR_NONFINITE : st;
+    }
     worst = std::max(worst, need);
     const long long m = std::min(max_sub, std::max(1ll, (long long)std::ceil(need)));
     DmdParams sub = prm;

@@ -147,6 +147,36 @@ def test_default_systems_keep_full_residuals(gpu_tables, name, prec, sub):
         assert np.array_equal(S.dmd_occupancy()[1], R.dmd_occupancy()[1])
 
 
+@pytest.mark.parametrize("variants", [None, (16 | 2, 16 | 1)], ids=["default", "pinned"])
+@pytest.mark.parametrize("prec", [btam.FP64, btam.FP32C])
+def test_results_of_a_refused_step(gpu_tables, prec, variants):
+    """A controlled step whose ratios are not finite ends with that error and
+    leaves the results of the evaluation it rests on: in full for a system left
+    to the defaults (bit for bit), its energies for pinned variants (to the
+    x-only test's tolerance of rho, V0 and S0 between the two forms)."""
+    s = cell()
+    S, R = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (S, R):
+        T.build_neighbors()
+        if variants:
+            T.set_variants(prec, *variants)
+    S.evaluate(prec)
+    S.dmd_setup()
+    S.set_state(sigma=s["sigma"] * 1.1)
+    with pytest.raises(btam.BtamError) as e:
+        S.dmd_step_ctl(2, prec, **dict(PRM, dt=1e308))
+    assert e.value.code == 6  # BTAM_ERR_NONFINITE
+    R.set_state(sigma=s["sigma"] * 1.1, x=S.dmd_occupancy()[0])
+    want = R.evaluate(prec)
+    got = S.results(want=tuple(want))
+    if variants is None:
+        for k, v in want.items():
+            assert np.array_equal(got[k], v), k
+    else:
+        for c in (0, 1):
+            assert abs(got["totals"][c] - want["totals"][c]) <= TOL[prec] * abs(want["totals"][c])
+
+
 def test_kept_values_are_bounded(gpu_tables):
     """Steps of a system whose kept values would exceed 4 GB leave no more than
     their small arrays in the library's pool (256 MB), and move as the general
