@@ -132,3 +132,24 @@ def test_totals_of_a_failed_relaxation(gpu_tables, relax):
     a, b = S.results(want=keys), R.results(want=keys)
     for k in keys:
         assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+def test_backtracked_trials(gpu_tables):
+    """A start far from a minimum, where the first trial of some iterations is
+    refused and halved: same evaluations, same iterates (the tolerance above; the
+    20 iterations carry a difference no further than that)."""
+    s = lattice.cluster("sphere", 8.0, x_fn=lambda g, r, n: g.uniform(0.0, 0.5, n),
+                        sigma_range=(0.03, 0.38), h_fraction=0.4, seed=2)
+    s["q"] = s["q"] + np.random.default_rng(2).normal(0.0, 0.25, s["q"].shape)
+    iters = 20
+    D, S = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (D, S):
+        T.build_neighbors()
+    want_q, want_s, want_F, evals = numpy_lbfgs(D, s, iters, 5)
+    assert evals > iters + 1
+    info = S.relax(mode=btam.RELAX_FP64, tol=1e-12, max_iter=iters, m=5)
+    q, sigma, _ = S.get_state()
+    assert info["iterations"] == iters and info["evaluations"] == evals
+    assert np.abs(q - want_q).max() <= 1e-9 * np.abs(want_q).max()
+    assert np.abs(sigma - want_s).max() <= 1e-9
+    assert abs(info["objective"] - want_F) <= 1e-10 * abs(want_F)
