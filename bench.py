@@ -61,7 +61,8 @@ NCU_L1_PIPE = {"pass1 pair-rule kernel": 0.90, "pass1 site kernel": 0.76,
 NCU_DRAM_BYTES_FP64 = {"pass1 pair-rule kernel": 263.3e6, "pass1 site kernel": 105.9e6,
                        "pass2 pair kernel": 487.4e6}
 # L1 data-pipe wavefront utilisation of the same FP64 launches (ncu
-# l1tex__data_pipe_lsu_wavefronts, share of peak): the binding unit
+# l1tex__data_pipe_lsu_wavefronts, share of peak): it binds the pair-rule
+# kernel; the latency of the gathers at 3-4 warps a scheduler binds the others
 NCU_L1_PIPE_FP64 = {"pass1 pair-rule kernel": 0.867, "pass1 site kernel": 0.644,
                     "pass2 pair kernel": 0.633}
 # shared-memory wavefronts per launch (trees and staged sums; the spline
@@ -861,7 +862,8 @@ def run_btam(args, ws, rank, local):
                               "dram_bytes_kernels": "pair-rule, pass-1 site and pass-2 pair kernels",
                               "algorithmic_bytes": 81 * n + 4 * P}
     roofline["l1_data_pipe"] = {
-        "bound": "L1 data pipe (random 32-byte halves of the 64-byte FP64 spline records)",
+        "bound": "L1 data pipe (random 32-byte halves of the 64-byte FP64 spline records) for "
+                 "the pair-rule kernel; gather latency at few resident warps for the others",
         "ncu_wavefront_frac": NCU_L1_PIPE_FP64,
         "source": "one ncu capture of the autotuned FP64 shapes (29, 30) on this workload"}
     roof32, und32 = kernel_roofline(prof32, shapes["fp32c"], fp32_peak, "fp32", NCU_DRAM_BYTES)
