@@ -2519,7 +2519,7 @@ static int dmd_controlled(btam_system *s, int precision, int nsteps, const doubl
     std::memcpy(r, bits, sizeof(r));
     const double need = std::max(r[0], r[1]);
     if (!std::isfinite(need)) {  // the call ends here, the results stay complete
-      st = residuals ? dmd_residuals(s, precision) : BTAM_OK;
+      st = dmd_residuals(s, precision);
       if (st == BTAM_OK) st = relax_totals(s);
       return st == BTAM_OK ? BTAM_ERR_NONFINITE : st;
     }

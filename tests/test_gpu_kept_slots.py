@@ -177,6 +177,24 @@ def test_results_of_a_refused_step(gpu_tables, prec, variants):
             assert abs(got["totals"][c] - want["totals"][c]) <= TOL[prec] * abs(want["totals"][c])
 
 
+@pytest.mark.parametrize("prec", [btam.FP64, btam.FP32C])
+def test_results_of_a_refused_run(gpu_tables, prec):
+    """The same in a run that would relax after its steps."""
+    s = cell()
+    S, R = btam.System(gpu_tables, s), btam.System(gpu_tables, s)
+    for T in (S, R):
+        T.build_neighbors()
+    S.dmd_setup()
+    with pytest.raises(btam.BtamError) as e:
+        S.dmd_run(2, prec, relax_every=1, relax_max_iter=2, **dict(PRM, dt=1e308))
+    assert e.value.code == 6
+    R.set_state(x=S.dmd_occupancy()[0])
+    want = R.evaluate(prec)
+    got = S.results(want=tuple(want))
+    for k, v in want.items():
+        assert np.array_equal(got[k], v), k
+
+
 def test_kept_values_are_bounded(gpu_tables):
     """Steps of a system whose kept values would exceed 4 GB leave no more than
     their small arrays in the library's pool (256 MB), and move as the general
