@@ -5,7 +5,7 @@
 // thread, as the slots of the result copies were (1 MB of pinned memory, five
 // events, a stream), it made 48 jobs on threads of their own, eight at a time,
 // take 95 ms where plain copies took 32 and where resources that are handed on
-// take 29.  So
+// take 27.  So
 //  * a thread that ends leaves its resource here, and the next that asks has it;
 //  * if none lies here, the first of the process is made at once; any other
 //    only for a thread that has asked kPatience times, since most threads that
